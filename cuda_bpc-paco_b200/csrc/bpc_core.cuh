@@ -55,7 +55,8 @@ constexpr uint32_t kSignTab = (0u << 0) | (2u << 3) | (3u << 6) | (4u << 9) | (6
 // out of a word of four, zero-extended, with the predicted sign (ctx & 1) in
 // bit 15 (which selects a zero byte either way).  Threads tid, tid + n, ...
 // fill it.
-constexpr uint32_t kSignBits = 0x00225522u, kSignHash = 0x01040400u;
+// The eight neighbours of a significance context are at kCtxBits.
+constexpr uint32_t kCtxBits = 0x00070507u, kSignBits = 0x00225522u, kSignHash = 0x01040400u;
 constexpr int kSignTableBytes = 512;
 BPC_FI void build_sign_table(uint8_t *table, int tid, int n) {
     uint16_t *t = reinterpret_cast<uint16_t *>(table);
@@ -132,8 +133,8 @@ struct Geo {
     static constexpr int NL = CBS / 2;                   // lanes per codeblock
     static constexpr int NG = 32 / NL;                   // codeblocks per warp
     static constexpr int CAP = CBS * CBS;                // slot size in ints
-    static constexpr int RING = CBS == 64 ? 512 : 256;   // decoder: codeword ring per codeblock
-    static constexpr int CHUNK = RING / 2;               // refill size
+    static constexpr int RING = CBS == 64 ? 512 : 256;   // decoder: codeword window per codeblock
+    static constexpr int CHUNK = RING / 2;               // words a refill moves the window on
     // decoder state of a warp in shared memory (bpc_dec.cuh): row bytes,
     // refinement sets, SPP-coded marks
     static constexpr int ROW_WORDS = CBS / 4 * 32, REF_WORDS = CBS / 16 * 32, VIS_WORDS = CBS / 4 * 8;
@@ -253,18 +254,19 @@ BPC_FI void count8(const uint64_t x[8], uint64_t &c0, uint64_t &c1, uint64_t &c2
 // (kEvOpen).
 constexpr int kEvKeys = 256, kEvOpen = 256, kEvVals = 257;
 
-// Decoder codeword ring refill: lane gl of a codeblock's lane group copies
-// its share of slot words [first, first + nwords) into the ring with 16-byte
-// loads; words past in_cap read as -1.  Kept out of line: it runs once per 256
-// codewords, and inlined into every decoder step body it would crowd the
-// instruction cache.
+// Decoder codeword window: lane gl of a codeblock's lane group fills its share
+// of the window with slot words [first, first + RING), 16-byte loads where it
+// can; words past in_cap read as -1.  (The words of the window's second half
+// move to its first half through memory again: they are in L2 or L1, and this
+// runs once per 256 codewords.)  Kept out of line: inlined into every decoder
+// step body it would crowd the instruction cache.
 template <int CBS>
 BPC_NOINLINE void ring_fill(uint32_t *ring, const int32_t *slot_in, uint32_t in_cap, bool compact, uint32_t first,
-                            int gl, int nwords) {
-    constexpr int NL = CBS / 2, RING = CBS == 64 ? 512 : 256;
-    const int per = nwords / NL;  // 8 or 16, multiple of 4
+                            int gl) {
+    using G = Geo<CBS>;
+    constexpr int per = G::RING / G::NL;  // 16, a multiple of 4
     for (int q = 0; q < per; q += 4) {
-        const uint32_t k = first + (uint32_t)(gl * per + q);
+        const uint32_t r = (uint32_t)(q * G::NL + 4 * gl), k = first + r;
         uint32_t v0, v1, v2, v3;
         if (k + 3 < in_cap && !compact) {
 #if defined(__CUDA_ARCH__)
@@ -285,7 +287,6 @@ BPC_NOINLINE void ring_fill(uint32_t *ring, const int32_t *slot_in, uint32_t in_
             v2 = k + 2 < in_cap ? (uint32_t)slot_in[k + 2] : 0xFFFFFFFFu;
             v3 = k + 3 < in_cap ? (uint32_t)slot_in[k + 3] : 0xFFFFFFFFu;
         }
-        const uint32_t r = k & (RING - 1);
         ring[r] = v0;
         ring[r + 1] = v1;
         ring[r + 2] = v2;

@@ -35,7 +35,7 @@ struct Coder<PASSES, CBS, false, W, LAT> {
     const Params &p;
     const uint8_t *tab;     // LUT bytes
     const uint16_t *sgtab;  // sign-context table (build_sign_table)
-    uint32_t *ring;         // codewords of this lane group's codeblock
+    uint32_t *ring;         // codeword window of this lane group's codeblock
     uint32_t *rowbase;      // row words of the warp, [row / 4][lane]
     uint32_t *rows;         // ... this lane's first one
     uint8_t *vis;           // 3 passes: own coefficients SPP coded in the plane, 2 bits a row, [row / 4][lane]
@@ -51,8 +51,9 @@ struct Coder<PASSES, CBS, false, W, LAT> {
     // arithmetic decoder: the interval [L - 1, E - 1] of the codeword cw; L ==
     // E when the codeword is used up
     uint32_t L, E, cw;
-    uint32_t cnt;      // codewords reserved in this codeblock (group-uniform)
-    uint32_t ring_hi;  // slot words [ring_hi - RING, ring_hi) are in the ring
+    // codeword window: slot words [first, first + RING), the next codeword at
+    // word pos of it (group-uniform)
+    uint32_t pos, first;
     bool anysig;       // some coefficient of the warp is significant (warp-uniform)
     int sig_base;      // LUT byte index of the current plane and pass
     uint32_t P4;       // its four sign probabilities, one per byte
@@ -76,25 +77,16 @@ struct Coder<PASSES, CBS, false, W, LAT> {
 
     // ---------------------------------------------------------------- AC
     // Lanes with an empty codeword take the next ones in lane order (:268-279);
-    // past the slot the ring holds the -1 fill (the overflow itself is reported
-    // once, from the final count, at the codeblock's end).  The ring is
-    // refilled here, where it is read, and not checked on steps that reserve
-    // nothing: it holds words up to cnt + NL for every reservation, and a
-    // refill replaces only words below cnt.
+    // past the slot the window holds the -1 fill (the overflow itself is
+    // reported once, from the final count, at the codeblock's end).
     BPC_FI void reserve(bool need, uint32_t ball) {
         const uint32_t bal = ball & gmask;
-        if (cnt + 1u + (uint32_t)G::NL > ring_hi) {  // group-uniform
-            w.syncmask(gmask);
-            ring_load(ring_hi, G::CHUNK);
-            ring_hi += G::CHUNK;
-            w.syncmask(gmask);
-        }
         if (need) {
-            cw = ring[(1u + cnt + (uint32_t)popc32(bal & ltmask)) & (G::RING - 1)];
+            cw = ring[pos + (uint32_t)popc32(bal & ltmask)];
             L = 1u;
             E = 0x10000u;
         }
-        cnt += (uint32_t)popc32(bal);
+        pos += (uint32_t)popc32(bal);
     }
 
     // Arithmetic_decoder :297-339.  With Lower = L - 1 and Size = E - L the
@@ -111,8 +103,20 @@ struct Coder<PASSES, CBS, false, W, LAT> {
         return act && sym;
     }
 
-    BPC_FI void ring_load(uint32_t first, int nwords) {
-        ring_fill<CBS>(ring, slot_in, in_cap, p.offsets != nullptr, first, gl, nwords);
+    // The codeword window: RING words of the slot from word `first` on, the
+    // next codeword at ring[pos].  Before CALLS coder calls (at most NL
+    // codewords each): once fewer words are left than those may take, the
+    // used ones are dropped and the window is filled up again.
+    template <int CALLS>
+    BPC_FI void ring_ensure() {
+        static_assert(CALLS * G::NL <= G::CHUNK, "");
+        if (pos > (uint32_t)(G::RING - CALLS * G::NL)) {  // group-uniform
+            w.syncmask(gmask);
+            ring_fill<CBS>(ring, slot_in, in_cap, p.offsets != nullptr, first + (uint32_t)G::CHUNK, gl);
+            pos -= (uint32_t)G::CHUNK;
+            first += (uint32_t)G::CHUNK;
+            w.syncmask(gmask);
+        }
     }
 
     // Decoder reconstruction: the reference ORs a plane mask 3 << b into the
@@ -122,17 +126,25 @@ struct Coder<PASSES, CBS, false, W, LAT> {
     // plane 0 is read back then).
 
     // ------------------------------------------------------------- contexts
+    template <int CC>
+    BPC_FI uint32_t sig_prob(uint32_t lo) const {
+        return tab[sig_base + popc32(lo & (kCtxBits << CC))];
+    }
+    // Compute_Sign_Context :178-226 over left, right, up and below
+    template <int CC>
+    BPC_FI uint32_t sign_entry(uint32_t lo) const {
+        return sgtab[((lo & (kSignBits << CC)) * (kSignHash >> CC)) >> 24];
+    }
+
     // One step: the coefficient of column CC in the row at byte 1 of lo.
-    // k8: CP, the row's coefficients SPP coded (bits 0, 1); SPP, collects them
-    // at bits 8, 9.
+    // k8: CP, the row's coefficients SPP coded, at their own bits of lo (9, 10);
+    // SPP, collects them at bits 8, 9.
     template <int PK, int CC>
-    BPC_FI void step(uint32_t &lo, uint32_t &k8, bool lowp, bool act) {
-        constexpr uint32_t kOwn = 0x200u << CC, kCtx = 0x070507u << CC;
-        const uint32_t nb = lo & kCtx;
-        bool coded = act && !(lo & kOwn);
-        if (PK == PK_CP) coded = coded && !(k8 & (1u << CC));
+    BPC_FI void step(uint32_t &lo, uint32_t &k8, bool act) {
+        constexpr uint32_t kOwn = 0x200u << CC, kNb = CC ? 0x100u : 0x800u;
+        bool coded = act && ((PK == PK_CP ? lo | k8 : lo) & kOwn) == 0u;
         if (PK == PK_SPP && PASSES == 3) {
-            coded = coded && nb != 0u;  // else it defers to CP (:450-452)
+            coded = coded && (lo & (kCtxBits << CC)) != 0u;  // else it defers to CP (:450-452)
             if (coded) k8 |= 0x100u << CC;
         }
         if (PK == PK_CP || PASSES == 3) {
@@ -140,32 +152,16 @@ struct Coder<PASSES, CBS, false, W, LAT> {
         }
         uint32_t sg = 0;
         if (LAT > 0) sg = sign_entry<CC>(lo);
-        const uint32_t P = tab[sig_base + popc32(nb)];
-        const bool sym = ac_dec(coded, P);
-        const bool ns = sym && lowp;
+        const bool ns = ac_dec(coded, sig_prob<CC>(lo));
         const uint32_t nsb = w.ballot(ns);
         if (!nsb) return;
+        // sign call of the lanes that became significant; the neighbour lane's
+        // copy of their byte follows from the ballots
+        const uint32_t nb_bit = CC ? bit_up : bit_dn;
         if (LAT == 0) sg = sign_entry<CC>(lo);
-        sign<CC>(lo, ns, nsb, sg);
-    }
-
-    // Compute_Sign_Context :178-226 over left, right, up and below
-    template <int CC>
-    BPC_FI uint32_t sign_entry(uint32_t lo) const {
-        return sgtab[((lo & (kSignBits << CC)) * (kSignHash >> CC)) >> 24];
-    }
-
-    // Sign call of the lanes that became significant, and the update of their
-    // own byte and of the neighbour lane's copy (two ballots, no shuffle).
-    template <int CC>
-    BPC_FI void sign(uint32_t &lo, bool ns, uint32_t nsb, uint32_t sg) {
-        anysig = true;
-        const uint32_t P2 = perm8(P4, sg);
-        const bool one = ac_dec(ns, P2);
+        const bool one = ac_dec(ns, perm8(P4, sg));
         const bool neg = ns && one != ((sg >> 15) != 0u);
         const uint32_t negb = w.ballot(neg);
-        constexpr uint32_t kOwn = 0x200u << CC, kNb = CC ? 0x100u : 0x800u;
-        const uint32_t nb_bit = CC ? bit_up : bit_dn;
         if (ns) lo |= kOwn;
         if (neg) lo |= kOwn << 4;
         if (nsb & nb_bit) lo |= kNb;
@@ -192,15 +188,35 @@ struct Coder<PASSES, CBS, false, W, LAT> {
         return true;
     }
 
+    // Planes 28..32 of an all-zero codeblock: a symbol cannot make a
+    // coefficient significant there (its data bit is one of the reference's
+    // flag bits, :523-530), so every one is coded with context 0.
+    BPC_FI void high_plane(uint32_t P, bool act) {
+#pragma unroll 1
+        for (int t = 0; t < 2 * CBS; t += 8) {
+            if (flat_rows(P, act)) continue;
+#pragma unroll 1
+            for (int k = 0; k < 8; k++) {
+                ring_ensure<1>();
+                (void)ac_dec(act, P);
+            }
+        }
+    }
+
     template <int PK>
-    BPC_FI void ctx_pass(int b, bool act) {
+    BPC_FI void ctx_pass(int b, bool act_) {
+        // one codeblock a warp: it is active whenever the pass is run
+        const bool act = G::NG == 1 || act_;
         const int off = PK == PK_CP ? p.cp_off : 0;
-        const bool lowp = b <= 27;
         sig_base = off + p.a_sig + (g + b) * 9;
         const uint8_t *sp = tab + (off + p.a_sign + (g + b) * 4);
         P4 = (uint32_t)sp[0] | ((uint32_t)sp[1] << 8) | ((uint32_t)sp[2] << 16) | ((uint32_t)sp[3] << 24);
         if (PK == PK_SPP && PASSES == 3 && !anysig) return;  // every coefficient defers
         const uint32_t P0 = tab[sig_base];
+        if (b > 27) {
+            high_plane(P0, act);
+            return;
+        }
         uint32_t cur = rows[0], last = 0u;
 #pragma unroll 1
         for (int q = 0; q < CBS / 4; q++) {
@@ -209,17 +225,19 @@ struct Coder<PASSES, CBS, false, W, LAT> {
                 if (flat_rows(P0, act)) continue;
             }
             uint32_t lo = (cur << 8) | last, hi = (cur >> 24) | (nxt << 8), out = 0u;
-            uint32_t k8 = PASSES == 3 && PK == PK_CP ? vis[q * 32] : 0u;
+            uint32_t k8 = PASSES == 3 && PK == PK_CP ? (uint32_t)vis[q * 32] << 9 : 0u;
 #pragma unroll 1
             for (int r = 0; r < 4; r++) {
-                step<PK, 0>(lo, k8, lowp, act);
-                step<PK, 1>(lo, k8, lowp, act);
+                ring_ensure<4>();  // two steps of up to two calls
+                step<PK, 0>(lo, k8, act);
+                step<PK, 1>(lo, k8, act);
                 lo = funnel_r(lo, hi, 8);
                 hi >>= 8;
                 out = (out >> 8) | (lo << 24);
                 k8 >>= 2;
             }
             rows[q * 32] = out;
+            if (!anysig) anysig = w.any(out != 0u);
             if (PASSES == 3 && PK == PK_SPP) vis[q * 32] = (uint8_t)k8;
             last = out >> 24;
             cur = nxt;
@@ -238,21 +256,25 @@ struct Coder<PASSES, CBS, false, W, LAT> {
     }
 
     // MRP_Decoder :608-629 over the coefficients significant at the plane's
-    // start; only the steps where some lane has one are run.
+    // start; only the steps where some lane has one are run.  (Letting each
+    // lane decode on its own until its codeword is used up, and ranking the
+    // waiting lanes by position, needs fewer votes but measured slower on the
+    // serial chain of one codeblock: 187 -> 202 us, 2 passes.)
     BPC_FI void mrp_pass(int b, bool act) {
+        if (b > 27) return;  // nothing can be significant
         const uint32_t P = tab[g + b];
-        const bool lowp = b <= 27;
 #pragma unroll 1
         for (int q = 0; q < CBS / 16; q++) {
-            const uint32_t R = act ? ref[q * 32] : 0u;
+            const uint32_t R = G::NG == 1 || act ? ref[q * 32] : 0u;
             uint32_t bits = 0;
             uint32_t u = anysig ? w.reduce_or(R) : 0u;
             while (u) {
                 const uint32_t bit = u & (0u - u);
                 u ^= bit;
+                ring_ensure<1>();
                 if (ac_dec((R & bit) != 0u, P)) bits |= bit;
             }
-            if (lowp) planes[b][q] = bits;
+            planes[b][q] = bits;
         }
     }
 
@@ -300,7 +322,8 @@ struct Coder<PASSES, CBS, false, W, LAT> {
         const int x = cbx * CBS + 2 * gl, y0 = cby * CBS;
         g = lut_group(p, x, y0);
         L = E = cw = 0u;
-        cnt = 0u;
+        pos = 1u;
+        first = 0u;
         status = 0;
         anysig = false;
         msb = -1;
@@ -319,10 +342,7 @@ struct Coder<PASSES, CBS, false, W, LAT> {
         }
         w.sync();  // the last codeblock's reads of the ring are over
         if (ok) {
-            ring_load(0u, G::RING);
-            ring_hi = G::RING;
-        } else {
-            ring_hi = 0x7fffffffu;
+            ring_fill<CBS>(ring, slot_in, in_cap, p.offsets != nullptr, 0u, gl);
         }
 #pragma unroll
         for (int q = 0; q < CBS / 4; q++) {
@@ -373,6 +393,7 @@ struct Coder<PASSES, CBS, false, W, LAT> {
                 transpose32(a);
                 write_rows(dst + (size_t)(16 * q) * (size_t)p.X, vec, a, own16(q, 5));
             }
+            const uint32_t cnt = first + pos - 1u;  // codewords reserved
             if (cnt >= cap) status |= ST_OVERFLOW;  // a reservation read past the slot
             if (p.counts && gl == 0) p.counts[cb] = (int)cnt;
         }
