@@ -48,6 +48,40 @@ struct GpuWarp {
     __device__ __forceinline__ void atomic_or(int *p, int v) { atomicOr(p, v); }
 };
 
+// The LUT as bytes in shared memory, zero-padded to tab_n; entries outside
+// 0..255 are flagged and read as 0.  Four entries per load and several loads in
+// flight per thread: a CTA starts with this, and one load after another it took
+// 10-15 us of a small image's time (one-warp CTAs, 6480 entries).
+__device__ __forceinline__ void stage_lut(const Params &p, uint8_t *tab) {
+    int bad = 0;
+    const bool vec = ((uintptr_t)p.lut & 15u) == 0u;
+    const int n4 = vec ? p.lut_n / 4 : 0;
+    const int4 *lut4 = reinterpret_cast<const int4 *>(p.lut);
+#pragma unroll 8
+    for (int k = (int)threadIdx.x; k < n4; k += (int)blockDim.x) {
+        int4 v = __ldg(lut4 + k);
+        if (((unsigned)v.x | (unsigned)v.y | (unsigned)v.z | (unsigned)v.w) > 255u) {
+            bad = 1;
+            v.x = (unsigned)v.x > 255u ? 0 : v.x;
+            v.y = (unsigned)v.y > 255u ? 0 : v.y;
+            v.z = (unsigned)v.z > 255u ? 0 : v.z;
+            v.w = (unsigned)v.w > 255u ? 0 : v.w;
+        }
+        reinterpret_cast<uchar4 *>(tab)[k] =
+            make_uchar4((unsigned char)v.x, (unsigned char)v.y, (unsigned char)v.z, (unsigned char)v.w);
+    }
+#pragma unroll 4
+    for (int k = 4 * n4 + (int)threadIdx.x; k < p.tab_n; k += (int)blockDim.x) {
+        int v = k < p.lut_n ? __ldg(p.lut + k) : 0;
+        if (v < 0 || v > 255) {
+            bad = 1;
+            v = 0;
+        }
+        tab[k] = (uint8_t)v;
+    }
+    if (bad && p.status) atomicOr(p.status, ST_LUT_RANGE);
+}
+
 // WARPS codeblock warps per CTA: kWarps, or 1 for decodes of at most half a wave
 // (their heaviest codeblocks then land on different SMs, see launch_t); the
 // register budget stays that of kMinCtas x kWarps resident warps per SM
@@ -60,16 +94,7 @@ __global__ void __launch_bounds__(WARPS * 32, (ENC ? kMinCtasEnc : kMinCtasDec) 
     if (heavy == 1) asm volatile("griddepcontrol.launch_dependents;");
     extern __shared__ __align__(16) unsigned char smem[];
     uint8_t *tab = smem;
-    int bad = 0;
-    for (int k = (int)threadIdx.x; k < p.tab_n; k += (int)blockDim.x) {
-        int v = k < p.lut_n ? __ldg(p.lut + k) : 0;
-        if (v < 0 || v > 255) {
-            bad = 1;
-            v = 0;
-        }
-        tab[k] = (uint8_t)v;
-    }
-    if (bad && p.status) atomicOr(p.status, ST_LUT_RANGE);
+    stage_lut(p, tab);
     uint8_t *sgtab = smem + p.tab_n;
     if (!ENC) build_sign_table(sgtab, (int)threadIdx.x, (int)blockDim.x);
     __syncthreads();
