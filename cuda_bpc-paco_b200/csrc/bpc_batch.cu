@@ -93,7 +93,9 @@ __global__ void k_lut_bytes(const int *lut, int lut_n, uint8_t *tab, int tab_n, 
 }
 
 // resident warps per SM the register budget is sized for, whatever the CTA shape
-constexpr int kResidentWarpsEnc = kMinCtasEnc * kWarps, kResidentWarpsDec = kMinCtasDec * kWarps;
+// (and the most a schedule may ask for)
+constexpr int kBatchCtasEnc = 4, kBatchCtasDec = 7;
+constexpr int kResidentWarpsEnc = kBatchCtasEnc * kWarps, kResidentWarpsDec = kBatchCtasDec * kWarps;
 
 // WARPS warps per CTA (2, 4 or 8: a tuning choice); `order` (may be null)
 // lists the items in the order the queue hands them out
@@ -113,7 +115,7 @@ __global__ void __launch_bounds__(WARPS * 32, (ENC ? kResidentWarpsEnc : kReside
     GpuWarpB w;
     uint32_t planes[28][4];
     uint8_t ev_key[ENC ? kEvKeys : 1];
-    uint32_t ev_val[ENC ? kEvVals : 1];
+    __align__(8) uint32_t ev_val[ENC ? kEvVals : 1];
     for (;;) {
         unsigned it = 0;
         if (w.lane() == 0) it = atomicAdd(head, 1u);
@@ -283,7 +285,7 @@ struct Batch {
     size_t scan_tmp_bytes = 0;
     int sms = 148;
     // schedule
-    int ctas_enc = kMinCtasEnc, ctas_dec = kMinCtasDec, per_item = 4, use_graph = 1;
+    int ctas_enc = kBatchCtasEnc, ctas_dec = kBatchCtasDec, per_item = 4, use_graph = 1;
     int warps_enc = kWarps, warps_dec = kWarps;  // warps per CTA: 2, 4 or 8
     int cost_enc = 0, cost_dec = 0;              // queue order: 0 coarse subbands first, 1 cost order
     int seq_enc = 0, seq_dec = 0;                // class kernels: 0 concurrent (forked streams), 1 one after another
@@ -777,15 +779,15 @@ int bpc_batch_tune(void *batch, const int *const *d_coeffs, int *d_compact, long
     };
     for (int it : items) {
         float te_best = 1e30f, td_best = 1e30f;
-        int ce = kMinCtasEnc, cd = kMinCtasDec;
-        for (int c = 1; c <= kMinCtasEnc; c++) {
+        int ce = kBatchCtasEnc, cd = kBatchCtasDec;
+        for (int c = 1; c <= kBatchCtasEnc; c++) {
             int rc = bpc_batch_set_schedule(batch, c, b->ctas_dec, it, b->use_graph);
             if (rc) return rc;
             float t;
             if ((rc = timed(true, t))) return rc;
             if (t < te_best) te_best = t, ce = c;
         }
-        for (int c = 2; c <= kMinCtasDec; c++) {
+        for (int c = 2; c <= kBatchCtasDec; c++) {
             int rc = bpc_batch_set_schedule(batch, ce, c, it, b->use_graph);
             if (rc) return rc;
             float t;

@@ -170,6 +170,15 @@ BPC_FI int ctz32(uint32_t x) {
     return __builtin_ctz(x);
 #endif
 }
+BPC_FI uint32_t brev32(uint32_t x) {
+#if defined(__CUDA_ARCH__)
+    return __brev(x);
+#else
+    uint32_t r = 0;
+    for (int k = 0; k < 32; k++) r |= ((x >> k) & 1u) << (31 - k);
+    return r;
+#endif
+}
 BPC_FI int clz32(uint32_t x) {
 #if defined(__CUDA_ARCH__)
     return __clz(x);
@@ -247,12 +256,11 @@ BPC_FI void count8(const uint64_t x[8], uint64_t &c0, uint64_t &c1, uint64_t &c2
     c3 = k5 & k6;
 }
 
-// Sizes of the encoder's per-lane event arrays.  ev_key holds one pass's
-// reservations: at most one per symbol call, and a lane makes at most two
-// calls per coefficient of its stripe (256 for 64x64, 128 for 32x32).  ev_val
-// has one more word, the value of a codeword reserved in an earlier pass
-// (kEvOpen).
-constexpr int kEvKeys = 256, kEvOpen = 256, kEvVals = 257;
+// Size of the encoder's per-lane event array (8-byte aligned): two words per
+// reservation of one pass.  There is at most one reservation per symbol call,
+// and a lane makes at most two calls per coefficient of its stripe (256 for
+// 64x64, 128 for 32x32).  kEvKeys: no second array is needed.
+constexpr int kEvKeys = 1, kEvVals = 512;
 
 // Decoder codeword window: lane gl of a codeblock's lane group fills its share
 // of the window with slot words [first, first + RING), 16-byte loads where it
@@ -305,14 +313,11 @@ BPC_FI uint64_t shfl_down64(W &w, uint64_t v) {
     return ((uint64_t)hi << 32) | lo;
 }
 
-// LAT selects the latency form of the per-lane loops, for launches whose time is
-// the serial chain of their heaviest codeblocks rather than the SMs' issue rate:
-// the encoder codes LAT + 1 positions per loop iteration (independent
-// extractions and table reads ahead of the sequential coder updates), the
-// decoder (any LAT > 0) reads a step's sign context before its significance
-// decision.  They execute more instructions per symbol; the bitstream is the
-// same.  LAT = 0 is the base form.  Coder<..., ENC = true> is in bpc_enc.cuh,
-// ENC = false in bpc_dec.cuh.
+// LAT > 0 selects the decoder's latency form, for launches whose time is the
+// serial chain of their heaviest codeblocks rather than the SMs' issue rate: a
+// step reads its sign context before its significance decision (more
+// instructions, the same bitstream).  The encoder has one form.
+// Coder<..., ENC = true> is in bpc_enc.cuh, ENC = false in bpc_dec.cuh.
 template <int PASSES, int CBS, bool ENC, class W, int LAT = 0>
 struct Coder;
 

@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(WARPS * 32, (ENC ? kMinCtasEnc : kMinCtasDec) 
     GpuWarp w;
     uint32_t planes[28][4];  // per-thread bitplanes (local memory, L1-resident)
     uint8_t ev_key[ENC ? kEvKeys : 1];
-    uint32_t ev_val[ENC ? kEvVals : 1];
+    __align__(8) uint32_t ev_val[ENC ? kEvVals : 1];
     // Walk: heavy 0, codeblocks cb_begin + slot*NG, grid-stride; heavy 1, the
     // order's unit `slot` if slot < heavy_n; heavy 2, the order's unit
     // heavy_n + slot, then the units past every warp slot's first one, each
@@ -268,20 +268,10 @@ template <int PASSES, int CBS, bool ENC>
 static cudaError_t launch_t(const Params &p, int grid, cudaStream_t st, bool lat) {
     using G = Geo<CBS>;
     const int warps_needed = (p.cb_end - p.cb_begin + G::NG - 1) / G::NG;
-    const long long resident = resident_warps(ENC, -1);
     if constexpr (ENC) {
-        // Encodes of at most two waves end with the serial chains of their
-        // heaviest codeblocks: the latency forms of the symbol loop, three
-        // positions per iteration within one wave (a 2048x2048 encode: 0.180
-        // -> 0.154 ms), two within two waves (4096x4096: 0.417 -> 0.412 ms;
-        // three there: 0.430).  Longer encodes are issue-bound and keep the
-        // form with fewer instructions.
-        if (lat && grid <= 0 && warps_needed <= resident)
-            return launch_w<PASSES, CBS, ENC, kWarps, 2>(p, grid, warps_needed, st);
-        if (lat && grid <= 0 && warps_needed <= 2 * resident)
-            return launch_w<PASSES, CBS, ENC, kWarps, 1>(p, grid, warps_needed, st);
         return launch_w<PASSES, CBS, ENC, kWarps, 0>(p, grid, warps_needed, st);
     } else {
+        const long long resident = resident_warps(ENC, -1);
         // A decode of at most half a wave of resident warps runs one warp per
         // CTA (consecutive CTAs go to different SMs, so its heaviest codeblocks,
         // the coarse subbands, neighbours in raster order, do not share an SM's

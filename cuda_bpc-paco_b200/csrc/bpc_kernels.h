@@ -5,19 +5,20 @@
 
 #include "bpc_core.cuh"
 
-#ifndef ENC_MIN_CTAS
-#define ENC_MIN_CTAS 4
-#endif
-
 namespace bpc {
 
 constexpr int kWarps = 4;  // warps (codeblocks) per CTA
-// CTAs per SM the register budget is sized for: the decoder steps its lanes
-// together and needs many warps to hide latency (7 x 4 warps, <= 72
-// registers); the encoder runs each lane's coder on its own and needs the
-// registers more than the warps.
+// CTAs per SM the register budget is sized for.  Decoder: 7 x 4 warps at 72
+// registers (a 16384x16384 3-pass decode at 6 / 7 / 8 CTAs: 5.17 / 4.87 / 4.81
+// ms, but a 4096x4096 one, one wave, 0.384 / 0.390 / 0.404 ms).  Encoder: 5 x 4
+// warps at 102 registers (4 / 5 / 6 CTAs: 4.48 / 4.13 / 4.06 ms at 16384x16384,
+// 0.160 / 0.160 / 0.182 ms at 2048x2048, where the 6-CTA form's spills lengthen
+// the serial chain of the heaviest codeblock).
 #ifndef DEC_MIN_CTAS
 #define DEC_MIN_CTAS 7
+#endif
+#ifndef ENC_MIN_CTAS
+#define ENC_MIN_CTAS 5
 #endif
 constexpr int kMinCtasDec = DEC_MIN_CTAS;
 constexpr int kMinCtasEnc = ENC_MIN_CTAS;
@@ -31,10 +32,10 @@ inline bool aligned_to(const void *p, unsigned a) { return ((uintptr_t)p & (uint
 
 // Launch the encoder (enc) or decoder over p.ncb codeblocks.  grid <= 0 picks
 // one CTA per kWarps codeblocks; a positive grid runs persistent CTAs that
-// walk the codeblocks grid-stride.  latency_forms lets a launch of a few waves
-// take the latency forms of the coder loops (and one-warp CTAs for a small
-// decode), which finish a launch alone on the GPU sooner but execute more
-// instructions; callers that run many launches at once pass false.
+// walk the codeblocks grid-stride.  latency_forms lets a decode of a few waves
+// take the latency form of the step (and one-warp CTAs if it is small), which
+// finishes a launch alone on the GPU sooner but executes more instructions;
+// callers that run many launches at once pass false.
 cudaError_t launch_code(bool enc, int passes, int cbs, const Params &p, int grid, cudaStream_t st,
                         bool latency_forms = true);
 

@@ -70,6 +70,27 @@ def test_unusual_probabilities(emu, oracle_mod, passes, cb, lo, hi):  # noqa: F8
         np.testing.assert_array_equal(dec.reshape(img.shape), wdec)
 
 
+@pytest.mark.parametrize("passes", [2, 3])
+@pytest.mark.parametrize("cb", [64, 32])
+def test_magnitudes_out_of_range(emu, oracle_mod, passes, cb):  # noqa: F811
+    """|x| >= 2^28 (MSB 28..31) is flagged and its codeblock marked with that
+    plane; the other codeblocks are coded as ever."""
+    img = bpc_synth.synthetic_coefficients(128, 5, 9, amp=30)
+    lut = oracle_mod.load_luts(lut_folder(passes), passes, 5)
+    want = oracle_mod.encode(img, lut, passes, 5, cb).reshape(-1, cb * cb)
+    bad = {}
+    for y, x, v in ((3, 5, 1 << 28), (70, 3, -(1 << 30)), (90, 100, -(1 << 31))):
+        img[y, x] = v
+        bad[y // cb * (128 // cb) + x // cb] = abs(v).bit_length() - 1
+    for kind in (0, 2, 3):
+        got, st = run(emu, 1, img, img.shape, lut, passes, 5, cb, kind=kind)
+        got = got.reshape(-1, cb * cb)
+        assert st == 4
+        assert {k: int(got[k, 0]) for k in bad} == bad
+        rest = [k for k in range(len(got)) if k not in bad]
+        np.testing.assert_array_equal(got[rest], want[rest])
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("cb", [64, 32])
 def test_decode_into_4_byte_aligned_raster(bpc, cb):
