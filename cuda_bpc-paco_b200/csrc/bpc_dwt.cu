@@ -8,12 +8,23 @@
 //   predict:  d[i] = x[2i+1] - floor((x[2i] + x[2i+2]) / 2)
 //   update:   s[i] = x[2i]   + floor((d[i-1] + d[i] + 2) / 4)
 //
-// Per level, forward: the row step reads the level's region from the data
-// raster and writes it to a scratch raster the caller provides, the column
-// step reads it back and writes the data raster (the inverse runs columns, then
-// rows).  Each step is one kernel in which a thread lifts a run of pairs of one
-// row (16-byte loads and stores) or one column (a warp covers 32 adjacent
-// columns, so every access is coalesced).
+// What bounds it: HBM traffic, and launches for small images.  One kernel does
+// a level, rows and columns: a thread walks down a strip of 8 columns (4
+// lifting pairs), lifts each row it reads in registers (the neighbours' samples
+// by shuffle) and keeps the column lifting's state of those 8 values, so a
+// level's region is read once and written once, with 16-byte accesses.  (A row
+// kernel and a column kernel through the scratch moved it twice.)
+//
+// In place.  A level writes its four quadrants over rows other threads still
+// read, so levels go out of place, in turn: level 1 data -> scratch, level 2
+// scratch -> data (its details are then where they belong), level 3 data ->
+// scratch, and so on; one copy kernel at the end brings the details of the odd
+// levels back.  The inverse starts with that copy, the other way, and ends with
+// level 1, scratch -> data.  Traffic per coefficient, 5 levels: 8 * 1.33 + 6.4
+// = 17 B instead of 21 B, and 6 launches instead of 10.  B200, 5 levels, forward
+// / inverse: 512x512 63 / 62 -> 35 / 35 us, 4096x4096 99 / 113 -> 72 / 66 us,
+// 8192x6144 204 / 225 -> 166 / 155 us, 16384x16384 917 / 945 -> 765 / 715 us (6.0 /
+// 6.4 TB/s over those 17 B).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -23,211 +34,252 @@
 
 namespace {
 
-// All four kernels work out of place (data -> scratch -> data per level), so
-// each level reads and writes its region exactly once per direction of the
-// row step and once for the column step.  A thread computes K consecutive
-// lifting pairs of one row (or column) from its own inputs plus a two-sample
-// halo on the left and one on the right; neighbouring threads read the halo
-// samples again, from L1.
-
-// forward, along a row: in[0, w) -> out[0, w/2) = s, out[w/2, w) = d
-template <int K>
-__global__ void k_rows_fwd(const int32_t *in, int32_t *out, long long stride, int w, int h) {
-    const int half = w >> 1;
-    const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) * K;
-    const int r = blockIdx.y;
-    if (i0 >= half || r >= h) return;
-    const int32_t *p = in + (long long)r * stride;
-    int32_t *q = out + (long long)r * stride;
-    int32_t x[2 * K + 1];
-    const bool vec = 2 * i0 + 2 * K < w && (((uintptr_t)(p + 2 * i0)) & 15) == 0 && K % 2 == 0;
-    if (vec) {
-#pragma unroll
-        for (int k = 0; k < 2 * K; k += 4) {
-            const int4 v = *reinterpret_cast<const int4 *>(p + 2 * i0 + k);
-            x[k] = v.x;
-            x[k + 1] = v.y;
-            x[k + 2] = v.z;
-            x[k + 3] = v.w;
-        }
-        x[2 * K] = p[2 * i0 + 2 * K];
-    } else {
-#pragma unroll
-        for (int k = 0; k <= 2 * K; k++) {
-            const int e = 2 * i0 + k;
-            x[k] = p[e < w ? e : w - 2];  // x[w] = x[w - 2]; samples past it are never used
-        }
-    }
-    int32_t dprev = 0;
-    if (i0 > 0) dprev = p[2 * i0 - 1] - ((p[2 * i0 - 2] + x[0]) >> 1);
-    int32_t sv[K], dv[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-        const int i = i0 + k;
-        const int32_t xn = 2 * i + 2 < w ? x[2 * k + 2] : x[2 * k];  // x[w] = x[w - 2]
-        const int32_t d = x[2 * k + 1] - ((x[2 * k] + xn) >> 1);
-        const int32_t dm = i == 0 ? d : dprev;
-        sv[k] = x[2 * k] + ((dm + d + 2) >> 2);
-        dv[k] = d;
-        dprev = d;
-    }
-    if (i0 + K <= half && (((uintptr_t)(q + i0)) & 15) == 0 && (((uintptr_t)(q + half + i0)) & 15) == 0 &&
-        K % 4 == 0) {
-#pragma unroll
-        for (int k = 0; k < K; k += 4) {
-            *reinterpret_cast<int4 *>(q + i0 + k) = make_int4(sv[k], sv[k + 1], sv[k + 2], sv[k + 3]);
-            *reinterpret_cast<int4 *>(q + half + i0 + k) = make_int4(dv[k], dv[k + 1], dv[k + 2], dv[k + 3]);
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < K; k++)
-            if (i0 + k < half) {
-                q[i0 + k] = sv[k];
-                q[half + i0 + k] = dv[k];
-            }
-    }
-}
-
-// V adjacent columns per thread, loaded and stored together (V = 4: 16-byte
-// accesses, a warp covers 128 columns of a row)
-template <int V>
-struct Cols {
-    int32_t v[V];
-};
-template <int V>
-__device__ __forceinline__ Cols<V> ld(const int32_t *p) {
-    Cols<V> r;
-    if constexpr (V == 4) {
-        const int4 t = *reinterpret_cast<const int4 *>(p);
-        r.v[0] = t.x, r.v[1] = t.y, r.v[2] = t.z, r.v[3] = t.w;
-    } else {
-#pragma unroll
-        for (int k = 0; k < V; k++) r.v[k] = p[k];
-    }
-    return r;
-}
-template <int V>
-__device__ __forceinline__ void st(int32_t *p, const Cols<V> &r) {
-    if constexpr (V == 4) {
-        *reinterpret_cast<int4 *>(p) = make_int4(r.v[0], r.v[1], r.v[2], r.v[3]);
-    } else {
-#pragma unroll
-        for (int k = 0; k < V; k++) p[k] = r.v[k];
-    }
-}
-
-// forward, along a column: rows [0, h) -> rows [0, h/2) = s, [h/2, h) = d
-template <int K, int V>
-__global__ void k_cols_fwd(const int32_t *in, int32_t *out, long long stride, int w, int h) {
-    const int c = (blockIdx.x * blockDim.x + threadIdx.x) * V;
-    const int half = h >> 1;
-    const int i0 = blockIdx.y * K;
-    if (c >= w || i0 >= half) return;
-    auto X = [&](int row) { return ld<V>(in + (long long)(row < h ? row : h - 2) * stride + c); };
-    Cols<V> dprev{}, xe = X(2 * i0);
-    if (i0 > 0) {
-        const Cols<V> a = X(2 * i0 - 2), b = X(2 * i0 - 1);
-#pragma unroll
-        for (int k = 0; k < V; k++) dprev.v[k] = b.v[k] - ((a.v[k] + xe.v[k]) >> 1);
-    }
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-        const int i = i0 + k;
-        if (i >= half) break;
-        const Cols<V> xn = X(2 * i + 2), xo = X(2 * i + 1);  // x[h] = x[h - 2]
-        Cols<V> sv, dv;
-#pragma unroll
-        for (int u = 0; u < V; u++) {
-            const int32_t d = xo.v[u] - ((xe.v[u] + xn.v[u]) >> 1);
-            const int32_t dm = i == 0 ? d : dprev.v[u];
-            sv.v[u] = xe.v[u] + ((dm + d + 2) >> 2);
-            dv.v[u] = d;
-        }
-        st<V>(out + (long long)i * stride + c, sv);
-        st<V>(out + (long long)(half + i) * stride + c, dv);
-        dprev = dv;
-        xe = xn;
-    }
-}
-
-// inverse, along a column: rows [0, h/2) = s, [h/2, h) = d -> rows [0, h)
-template <int K, int V>
-__global__ void k_cols_inv(const int32_t *in, int32_t *out, long long stride, int w, int h) {
-    const int c = (blockIdx.x * blockDim.x + threadIdx.x) * V;
-    const int half = h >> 1;
-    const int i0 = blockIdx.y * K;
-    if (c >= w || i0 >= half) return;
-    auto S = [&](int i) { return ld<V>(in + (long long)i * stride + c); };
-    auto D = [&](int i) { return ld<V>(in + (long long)(half + i) * stride + c); };
-    Cols<V> di = D(i0), e, s0 = S(i0), dm = i0 ? D(i0 - 1) : di;
-#pragma unroll
-    for (int u = 0; u < V; u++) e.v[u] = s0.v[u] - ((dm.v[u] + di.v[u] + 2) >> 2);
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-        const int i = i0 + k;
-        if (i >= half) break;
-        Cols<V> en = e, dn = di;
-        if (i + 1 < half) {  // x[h] = x[h - 2] at the end
-            dn = D(i + 1);
-            const Cols<V> sn = S(i + 1);
-#pragma unroll
-            for (int u = 0; u < V; u++) en.v[u] = sn.v[u] - ((di.v[u] + dn.v[u] + 2) >> 2);
-        }
-        Cols<V> odd;
-#pragma unroll
-        for (int u = 0; u < V; u++) odd.v[u] = di.v[u] + ((e.v[u] + en.v[u]) >> 1);
-        st<V>(out + (long long)(2 * i) * stride + c, e);
-        st<V>(out + (long long)(2 * i + 1) * stride + c, odd);
-        e = en;
-        di = dn;
-    }
-}
-
-// inverse, along a row: [0, w/2) = s, [w/2, w) = d -> [0, w)
-template <int K>
-__global__ void k_rows_inv(const int32_t *in, int32_t *out, long long stride, int w, int h) {
-    const int half = w >> 1;
-    const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) * K;
-    const int r = blockIdx.y;
-    if (i0 >= half || r >= h) return;
-    const int32_t *p = in + (long long)r * stride;
-    int32_t *q = out + (long long)r * stride;
-    int32_t di = p[half + i0];
-    int32_t e = p[i0] - (((i0 ? p[half + i0 - 1] : di) + di + 2) >> 2);
-    int32_t xv[2 * K];
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-        const int i = i0 + k;
-        int32_t en = e, dn = di;
-        if (i + 1 < half) {
-            dn = p[half + i + 1];
-            en = p[i + 1] - ((di + dn + 2) >> 2);
-        }
-        xv[2 * k] = e;
-        xv[2 * k + 1] = di + ((e + en) >> 1);
-        e = en;
-        di = dn;
-    }
-    if (2 * i0 + 2 * K <= w && (((uintptr_t)(q + 2 * i0)) & 15) == 0 && K % 2 == 0) {
-#pragma unroll
-        for (int k = 0; k < 2 * K; k += 4)
-            *reinterpret_cast<int4 *>(q + 2 * i0 + k) = make_int4(xv[k], xv[k + 1], xv[k + 2], xv[k + 3]);
-    } else {
-#pragma unroll
-        for (int k = 0; k < 2 * K; k++)
-            if (2 * i0 + k < w) q[2 * i0 + k] = xv[k];
-    }
-}
-
-// 16-byte column accesses: both rasters 16-byte aligned, row stride and level
-// width multiples of 4 ints
-bool vec4(const int *a, const int *b, int stride, int w) {
-    return ((((uintptr_t)a) | ((uintptr_t)b)) & 15) == 0 && stride % 4 == 0 && w % 4 == 0;
-}
-
-constexpr int kRowPairs = 4;   // lifting pairs per thread along a row
-constexpr int kColPairs = 8;   // ... along a column
 constexpr int kThreads = 128;
+constexpr unsigned kFull = 0xffffffffu;
+
+// Vertical pairs per thread.  A strip reads 3 rows above its own again (from L2:
+// its neighbour reads them at the same time); longer strips re-read less but
+// leave the GPU idle at small levels (512x512 / 8192x6144 / 16384x16384 forward,
+// 5 levels: 1 pair 36 / 168 / 793 us, 2: 35 / 166 / 765, 4: 40 / 172 / 773, 16,
+// before chained launches: 91 / 231 / 796).
+constexpr int kPairs = 2;
+
+
+// Lets the next kernel of the call become resident, and waits for the one
+// before to complete (returns at once in a plain launch).
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <int N>
+__device__ __forceinline__ void load_run(const int32_t *p, int32_t *v) {
+    if constexpr (N % 4 == 0) {
+#pragma unroll
+        for (int k = 0; k < N; k += 4) {
+            const int4 t = *reinterpret_cast<const int4 *>(p + k);
+            v[k] = t.x, v[k + 1] = t.y, v[k + 2] = t.z, v[k + 3] = t.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < N; k++) v[k] = p[k];
+    }
+}
+template <int N>
+__device__ __forceinline__ void store_run(int32_t *p, const int32_t *v) {
+    if constexpr (N % 4 == 0) {
+#pragma unroll
+        for (int k = 0; k < N; k += 4)
+            *reinterpret_cast<int4 *>(p + k) = make_int4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < N; k++) p[k] = v[k];
+    }
+}
+
+// P lifting pairs of a row per thread: 4 (16-byte accesses) or 1.  The strip
+// starts at column c = 2 P (thread); lanes past the row's end (on = false) take
+// part in the shuffles only.  v: the P low values, then the P high ones.
+template <int P>
+__device__ __forceinline__ void lift_row(const int32_t *row, int c, int w, bool on, int lane, int32_t v[2 * P]) {
+    int32_t x[2 * P] = {}, xn = 0, xa = 0, xb = 0;
+    if (on) {
+        load_run<2 * P>(row + c, x);
+        if (lane == 31 && c + 2 * P < w) xn = row[c + 2 * P];
+        if (lane == 0 && c > 0) xa = row[c - 2], xb = row[c - 1];
+    }
+    const int32_t nb = __shfl_down_sync(kFull, x[0], 1);
+    if (lane != 31) xn = nb;
+    if (c + 2 * P >= w) xn = x[2 * P - 2];  // x[w] = x[w - 2]
+    int32_t d[P];
+#pragma unroll
+    for (int k = 0; k < P; k++) d[k] = x[2 * k + 1] - ((x[2 * k] + (k + 1 < P ? x[2 * k + 2 < 2 * P ? 2 * k + 2 : 0] : xn)) >> 1);
+    int32_t dp = __shfl_up_sync(kFull, d[P - 1], 1);
+    if (lane == 0) dp = xb - ((xa + x[0]) >> 1);
+    if (c == 0) dp = d[0];
+#pragma unroll
+    for (int k = 0; k < P; k++) {
+        v[k] = x[2 * k] + ((dp + d[k] + 2) >> 2);
+        v[P + k] = d[k];
+        dp = d[k];
+    }
+}
+
+// One level, rows then columns: the top-left w x h of `in` to the four
+// quadrants of `out`, vertical pairs [blockIdx.y * kPairs, ...) per thread.
+template <int P>
+__global__ void __launch_bounds__(kThreads) k_fwd(const int32_t *in, int32_t *out, long long stride, int w, int h) {
+    after_previous();
+    const int c = (int)(blockIdx.x * kThreads + threadIdx.x) * 2 * P, lane = (int)(threadIdx.x & 31u);
+    const bool on = c < w;
+    const int hw = w >> 1, hh = h >> 1;
+    const int i0 = (int)blockIdx.y * kPairs, i1 = i0 + kPairs < hh ? i0 + kPairs : hh;
+    int32_t e[2 * P], dp[2 * P];  // row 2i, and the high values of pair i - 1
+    if (i0 > 0) {
+        int32_t a[2 * P], b[2 * P];
+        lift_row<P>(in + (long long)(2 * i0 - 2) * stride, c, w, on, lane, a);
+        lift_row<P>(in + (long long)(2 * i0 - 1) * stride, c, w, on, lane, b);
+        lift_row<P>(in + (long long)(2 * i0) * stride, c, w, on, lane, e);
+#pragma unroll
+        for (int k = 0; k < 2 * P; k++) dp[k] = b[k] - ((a[k] + e[k]) >> 1);
+    } else {
+        lift_row<P>(in, c, w, on, lane, e);
+    }
+    int32_t *lo = out + (long long)i0 * stride + (c >> 1), *hi = lo + (long long)hh * stride;
+#pragma unroll
+    for (int i = i0; i < i1; i++) {
+        int32_t o[2 * P], n[2 * P];
+        lift_row<P>(in + (long long)(2 * i + 1) * stride, c, w, on, lane, o);
+        if (2 * i + 2 < h) {
+            lift_row<P>(in + (long long)(2 * i + 2) * stride, c, w, on, lane, n);
+        } else {  // x[h] = x[h - 2]
+#pragma unroll
+            for (int k = 0; k < 2 * P; k++) n[k] = e[k];
+        }
+        int32_t s[2 * P], d[2 * P];
+#pragma unroll
+        for (int k = 0; k < 2 * P; k++) {
+            d[k] = o[k] - ((e[k] + n[k]) >> 1);
+            s[k] = e[k] + (((i == 0 ? d[k] : dp[k]) + d[k] + 2) >> 2);
+            dp[k] = d[k];
+            e[k] = n[k];
+        }
+        if (on) {
+            store_run<P>(lo, s);
+            store_run<P>(lo + hw, s + P);
+            store_run<P>(hi, d);
+            store_run<P>(hi + hw, d + P);
+        }
+        lo += stride;
+        hi += stride;
+    }
+}
+
+// One level back, columns then rows: the four quadrants of `in` to the top-left
+// w x h of `out`.  The rows need values of the strips to the left and right
+// that only come out of their column lifting, so the first and last lane of a
+// warp work for their neighbours and store nothing (30 strips per warp).
+template <int P>
+__global__ void __launch_bounds__(kThreads) k_inv(const int32_t *in, int32_t *out, long long stride, int w, int h) {
+    after_previous();
+    const int lane = (int)(threadIdx.x & 31u);
+    const int t = (int)(blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * 30 + lane - 1;
+    const int c = t * 2 * P;
+    const bool on = c >= 0 && c < w, mine = on && lane > 0 && lane < 31;
+    const int hw = w >> 1, hh = h >> 1;
+    const int i0 = (int)blockIdx.y * kPairs, i1 = i0 + kPairs < hh ? i0 + kPairs : hh;
+    const int32_t *lo = in + (c >> 1), *hi = lo + (long long)hh * stride;
+    auto low = [&](int i, int32_t v[2 * P]) {
+        if (!on) return;
+        load_run<P>(lo + (long long)i * stride, v);
+        load_run<P>(lo + (long long)i * stride + hw, v + P);
+    };
+    auto high = [&](int i, int32_t v[2 * P]) {
+        if (!on) return;
+        load_run<P>(hi + (long long)i * stride, v);
+        load_run<P>(hi + (long long)i * stride + hw, v + P);
+    };
+    auto put_row = [&](int r, const int32_t v[2 * P]) {  // v: P low values, P high ones
+        int32_t x[2 * P];
+        int32_t dm = __shfl_up_sync(kFull, v[2 * P - 1], 1);
+        if (c == 0) dm = v[P];
+#pragma unroll
+        for (int k = 0; k < P; k++) {
+            x[2 * k] = v[k] - ((dm + v[P + k] + 2) >> 2);
+            dm = v[P + k];
+        }
+        int32_t en = __shfl_down_sync(kFull, x[0], 1);
+        if (c + 2 * P >= w) en = x[2 * P - 2];  // x[w] = x[w - 2]
+#pragma unroll
+        for (int k = 0; k < P; k++)
+            x[2 * k + 1] = v[P + k] + ((x[2 * k] + (k + 1 < P ? x[2 * k + 2 < 2 * P ? 2 * k + 2 : 0] : en)) >> 1);
+        if (mine) store_run<2 * P>(out + (long long)r * stride + c, x);
+    };
+    int32_t e[2 * P] = {}, d[2 * P] = {}, dm[2 * P] = {};
+    low(i0, e);
+    high(i0, d);
+    if (i0 > 0) high(i0 - 1, dm);
+#pragma unroll
+    for (int k = 0; k < 2 * P; k++) e[k] -= ((i0 > 0 ? dm[k] : d[k]) + d[k] + 2) >> 2;
+#pragma unroll
+    for (int i = i0; i < i1; i++) {
+        int32_t en[2 * P] = {}, dn[2 * P] = {}, o[2 * P];
+        const bool more = i + 1 < hh;
+        if (more) {
+            low(i + 1, en);
+            high(i + 1, dn);
+        }
+#pragma unroll
+        for (int k = 0; k < 2 * P; k++) {
+            en[k] = more ? en[k] - ((d[k] + dn[k] + 2) >> 2) : e[k];  // x[h] = x[h - 2]
+            o[k] = d[k] + ((e[k] + en[k]) >> 1);
+        }
+        put_row(2 * i, e);
+        put_row(2 * i + 1, o);
+#pragma unroll
+        for (int k = 0; k < 2 * P; k++) e[k] = en[k], d[k] = dn[k];
+    }
+}
+
+// The details of levels 1, 3, ... (and, with whole, the low band of level
+// `levels`) from one raster to the other.  blockIdx.y counts row groups of
+// level 1, then of level 3, and so on.
+constexpr int kCopyRows = 4;
+template <int V>
+__global__ void __launch_bounds__(kThreads) k_copy_odd(const int32_t *in, int32_t *out, long long stride, int X, int Y, int levels) {
+    after_previous();
+    int y = (int)blockIdx.y, l = 1;
+    for (; l <= levels; l += 2) {
+        const int groups = ((Y >> (l - 1)) + kCopyRows - 1) / kCopyRows;
+        if (y < groups) break;
+        y -= groups;
+    }
+    const int w = X >> (l - 1), h = Y >> (l - 1);
+    const int c = (int)(blockIdx.x * kThreads + threadIdx.x) * V;
+    if (l > levels || c >= w) return;
+    int32_t v[kCopyRows][V];
+    bool on[kCopyRows];
+#pragma unroll
+    for (int k = 0; k < kCopyRows; k++) {
+        const int r = y * kCopyRows + k;
+        // the low quadrant belongs to the next level, unless this is the last
+        on[k] = r < h && (l == levels || r >= (h >> 1) || c >= (w >> 1));
+        if (on[k]) load_run<V>(in + (long long)r * stride + c, v[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < kCopyRows; k++)
+        if (on[k]) store_run<V>(out + (long long)(y * kCopyRows + k) * stride + c, v[k]);
+}
+
+// 16-byte accesses: both rasters 16-byte aligned, row stride and half a level's
+// width multiples of 4 ints
+bool vec4(const int *a, const int *b, int stride, int half) {
+    return ((((uintptr_t)a) | ((uintptr_t)b)) & 15) == 0 && stride % 4 == 0 && half % 4 == 0;
+}
+
+// Launch in stream order behind the level before it: its CTAs may become
+// resident while that one drains and wait for it at their start
+// (griddepcontrol.wait), which hides most of the launch latency (512x512 forward
+// 46 -> 35 us, 8192x6144 175 -> 166 us).
+template <class... P, class... A>
+cudaError_t launch(bool chained, dim3 grid, cudaStream_t st, void (*kernel)(P...), A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = chained ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    if (e == cudaErrorNotSupported && cfg.numAttrs) {  // plain stream order then
+        (void)cudaGetLastError();
+        cfg.numAttrs = 0;
+        e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    }
+    return e;
+}
 
 int check(cudaError_t e, const char *what) {
     if (e != cudaSuccess) {
@@ -244,6 +296,30 @@ bool valid(const int *d, const int *t, int X, int Y, int levels) {
            (X >> (levels ? levels - 1 : 0)) >= 2 && (Y >> (levels ? levels - 1 : 0)) >= 2 && X <= 32768 && Y <= 65535;
 }
 
+int level(bool fwd, bool chained, const int *in, int *out, int X, int Y, int l, cudaStream_t st) {
+    const int w = X >> (l - 1), h = Y >> (l - 1);
+    const unsigned gy = (unsigned)((h / 2 + kPairs - 1) / kPairs);
+    const bool vec = vec4(in, out, X, w / 2);
+    const int strips = vec ? w / 8 : w / 2, per = fwd ? kThreads : 30 * (kThreads / 32);
+    const dim3 g((unsigned)((strips + per - 1) / per), gy);
+    return check(launch(chained, g, st, fwd ? (vec ? k_fwd<4> : k_fwd<1>) : (vec ? k_inv<4> : k_inv<1>), in, out,
+                        (long long)X, w, h),
+                 "launch");
+}
+
+int copy_odd(bool chained, const int *in, int *out, int X, int Y, int levels, cudaStream_t st) {
+    unsigned gy = 0;
+    bool vec = true;
+    for (int l = 1; l <= levels; l += 2) {
+        gy += (unsigned)(((Y >> (l - 1)) + kCopyRows - 1) / kCopyRows);
+        vec = vec && vec4(in, out, X, (X >> (l - 1)) / 2);
+    }
+    const int per = kThreads * (vec ? 4 : 1);
+    const dim3 g((unsigned)((X + per - 1) / per), gy);
+    return check(launch(chained, g, st, vec ? k_copy_odd<4> : k_copy_odd<1>, in, out, (long long)X, X, Y, levels),
+                 "launch");
+}
+
 }  // namespace
 
 extern "C" {
@@ -251,38 +327,22 @@ extern "C" {
 int bpc_dwt53_forward(int *d_data, int X, int Y, int levels, int *d_tmp, void *stream) {
     if (!valid(d_data, d_tmp, X, Y, levels)) return BPC_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
-    for (int l = 0; l < levels; l++) {
-        const int w = X >> l, h = Y >> l;
-        const dim3 gr((unsigned)((w / 2 + kThreads * kRowPairs - 1) / (kThreads * kRowPairs)), (unsigned)h);
-        k_rows_fwd<kRowPairs><<<gr, kThreads, 0, st>>>(d_data, d_tmp, X, w, h);
-        if (vec4(d_data, d_tmp, X, w)) {
-            const dim3 gc((unsigned)((w / 4 + kThreads - 1) / kThreads), (unsigned)((h / 2 + kColPairs - 1) / kColPairs));
-            k_cols_fwd<kColPairs, 4><<<gc, kThreads, 0, st>>>(d_tmp, d_data, X, w, h);
-        } else {
-            const dim3 gc((unsigned)((w + kThreads - 1) / kThreads), (unsigned)((h / 2 + kColPairs - 1) / kColPairs));
-            k_cols_fwd<kColPairs, 1><<<gc, kThreads, 0, st>>>(d_tmp, d_data, X, w, h);
-        }
-        const int rc = check(cudaGetLastError(), "launch");
+    for (int l = 1; l <= levels; l++) {
+        const int rc = level(true, l > 1, l % 2 ? d_data : d_tmp, l % 2 ? d_tmp : d_data, X, Y, l, st);
         if (rc) return rc;
     }
-    return BPC_OK;
+    return levels ? copy_odd(true, d_tmp, d_data, X, Y, levels, st) : BPC_OK;
 }
 
 int bpc_dwt53_inverse(int *d_data, int X, int Y, int levels, int *d_tmp, void *stream) {
     if (!valid(d_data, d_tmp, X, Y, levels)) return BPC_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
-    for (int l = levels - 1; l >= 0; l--) {
-        const int w = X >> l, h = Y >> l;
-        if (vec4(d_data, d_tmp, X, w)) {
-            const dim3 gc((unsigned)((w / 4 + kThreads - 1) / kThreads), (unsigned)((h / 2 + kColPairs - 1) / kColPairs));
-            k_cols_inv<kColPairs, 4><<<gc, kThreads, 0, st>>>(d_data, d_tmp, X, w, h);
-        } else {
-            const dim3 gc((unsigned)((w + kThreads - 1) / kThreads), (unsigned)((h / 2 + kColPairs - 1) / kColPairs));
-            k_cols_inv<kColPairs, 1><<<gc, kThreads, 0, st>>>(d_data, d_tmp, X, w, h);
-        }
-        const dim3 gr((unsigned)((w / 2 + kThreads * kRowPairs - 1) / (kThreads * kRowPairs)), (unsigned)h);
-        k_rows_inv<kRowPairs><<<gr, kThreads, 0, st>>>(d_tmp, d_data, X, w, h);
-        const int rc = check(cudaGetLastError(), "launch");
+    if (levels) {
+        const int rc = copy_odd(false, d_data, d_tmp, X, Y, levels, st);
+        if (rc) return rc;
+    }
+    for (int l = levels; l >= 1; l--) {
+        const int rc = level(false, true, l % 2 ? d_tmp : d_data, l % 2 ? d_data : d_tmp, X, Y, l, st);
         if (rc) return rc;
     }
     return BPC_OK;
