@@ -72,6 +72,27 @@ BPC_FI void build_sign_table(uint8_t *table, int tid, int n) {
     }
 }
 
+// Eight 0-symbols of probability P from interval size sz: the size after them,
+// and before the last one (0: the codeword was used up before).
+BPC_FI void zero_run(uint32_t &sz, uint32_t &prev, uint32_t P) {
+    prev = sz;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        prev = sz;
+        sz = (sz * P) >> 7;
+    }
+}
+// 0-symbols until size sz is used up, at most 8
+BPC_FI int zero_count(uint32_t sz, uint32_t P) {
+    int n = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        n += sz != 0u ? 1 : 0;
+        sz = (sz * P) >> 7;
+    }
+    return n;
+}
+
 struct Params {
     const int32_t *in;   // encode: raster coefficients; decode: slot stream
     int32_t *out;        // encode: slot stream; decode: raster coefficients

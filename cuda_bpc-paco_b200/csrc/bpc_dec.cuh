@@ -92,15 +92,19 @@ struct Coder<PASSES, CBS, false, W, LAT> {
     // Arithmetic_decoder :297-339.  With Lower = L - 1 and Size = E - L the
     // reference's Lower + (Size * P >> 7) + 1 is the threshold below, and both
     // outcomes move one end of the interval to it.
-    BPC_FI bool ac_dec(bool act, uint32_t P) {
-        const bool need = act && L == E;
-        const uint32_t ball = w.ballot(need);
-        if (ball) reserve(need, ball);  // warp-uniform
+    BPC_FI bool ac_step(bool act, uint32_t P) {
         const uint32_t thr = L + (((E - L) * P) >> 7);
         const bool sym = cw >= thr;
         if (act && sym) L = thr + 1u;
         if (act && !sym) E = thr;
         return act && sym;
+    }
+    template <bool ALWAYS = false>  // reserve without a branch (that nobody reserves is rare)
+    BPC_FI bool ac_dec(bool act, uint32_t P) {
+        const bool need = act && L == E;
+        const uint32_t ball = w.ballot(need);
+        if (ALWAYS || ball) reserve(need, ball);  // warp-uniform
+        return ac_step(act, P);
     }
 
     // The codeword window: RING words of the slot from word `first` on, the
@@ -140,51 +144,112 @@ struct Coder<PASSES, CBS, false, W, LAT> {
     // k8: CP, the row's coefficients SPP coded, at their own bits of lo (9, 10);
     // SPP, collects them at bits 8, 9.
     template <int PK, int CC>
-    BPC_FI void step(uint32_t &lo, uint32_t &k8, bool act) {
-        constexpr uint32_t kOwn = 0x200u << CC, kNb = CC ? 0x100u : 0x800u;
-        bool coded = act && ((PK == PK_CP ? lo | k8 : lo) & kOwn) == 0u;
+    BPC_FI bool coded_here(uint32_t win, uint32_t &k8, bool act) {
+        bool coded = act && ((PK == PK_CP ? win | k8 : win) & (0x200u << CC)) == 0u;
         if (PK == PK_SPP && PASSES == 3) {
-            coded = coded && (lo & (kCtxBits << CC)) != 0u;  // else it defers to CP (:450-452)
+            coded = coded && (win & (kCtxBits << CC)) != 0u;  // else it defers to CP (:450-452)
             if (coded) k8 |= 0x100u << CC;
         }
+        return coded;
+    }
+    // the coefficients that became significant (ns, and their ballot) in this
+    // lane's byte; the neighbour lane's copy follows from the ballot
+    template <int CC>
+    BPC_FI void mark(uint32_t &win, bool ns, uint32_t nsb, int shift) {
+        if (ns) win |= (0x200u << CC) << shift;
+        if (nsb & (CC ? bit_up : bit_dn)) win |= (CC ? 0x100u : 0x800u) << shift;
+    }
+
+    template <int PK, int CC>
+    BPC_FI void step(uint32_t &lo, uint32_t &k8, bool act) {
+        const bool coded = coded_here<PK, CC>(lo, k8, act);
         if (PK == PK_CP || PASSES == 3) {
             if (!w.any(coded)) return;
         }
-        uint32_t sg = 0;
-        if (LAT > 0) sg = sign_entry<CC>(lo);
         const bool ns = ac_dec(coded, sig_prob<CC>(lo));
         const uint32_t nsb = w.ballot(ns);
         if (!nsb) return;
-        // sign call of the lanes that became significant; the neighbour lane's
-        // copy of their byte follows from the ballots
-        const uint32_t nb_bit = CC ? bit_up : bit_dn;
-        if (LAT == 0) sg = sign_entry<CC>(lo);
+        const uint32_t sg = sign_entry<CC>(lo);
         const bool one = ac_dec(ns, perm8(P4, sg));
         const bool neg = ns && one != ((sg >> 15) != 0u);
         const uint32_t negb = w.ballot(neg);
-        if (ns) lo |= kOwn;
-        if (neg) lo |= kOwn << 4;
-        if (nsb & nb_bit) lo |= kNb;
-        if (negb & nb_bit) lo |= kNb << 4;
+        mark<CC>(lo, ns, nsb, 0);
+        mark<CC>(lo, neg, negb, 4);
+    }
+
+    // The latency form.  On an SM with little else to run an ALU operation
+    // takes 5 cycles, a compare and a select on it 19, a compare, a vote and a
+    // branch on that 46, so the votes are taken in pairs, the sign context is
+    // read before the decision, and cx, a copy of lo whose significance bits
+    // are complete before the sign call, keeps the next step's context from
+    // waiting for this one's signs (one LL codeblock alone, 3 passes: 261 ->
+    // 256 us; with MRP reserving without a branch 250 us).
+    template <int PK, int CC>
+    BPC_FI void step_lat(uint32_t &lo, uint32_t &cx, uint32_t &k8, bool act) {
+        const bool coded = coded_here<PK, CC>(cx, k8, act);
+        bool need = coded && L == E;
+        uint32_t ball = w.ballot(need);
+        if (PK == PK_CP || PASSES == 3) {
+            if (!w.any(coded)) return;
+        }
+        const uint32_t sg = sign_entry<CC>(lo);
+        if (ball) reserve(need, ball);
+        const bool ns = ac_step(coded, sig_prob<CC>(cx));
+        const uint32_t nsb = w.ballot(ns);
+        need = ns && L == E;
+        ball = w.ballot(need);
+        if (!nsb) return;
+        mark<CC>(cx, ns, nsb, 0);
+        if (ball) reserve(need, ball);
+        const bool one = ac_step(ns, perm8(P4, sg));
+        const bool neg = ns && one != ((sg >> 15) != 0u);
+        const uint32_t negb = w.ballot(neg);
+        mark<CC>(lo, ns, nsb, 0);
+        mark<CC>(lo, neg, negb, 4);
     }
 
     // Four rows (eight steps) of a codeblock in which nothing is significant
     // yet: every coefficient is coded with context 0, and while all symbols
     // are 0 only E moves, down the same chain whatever the codeword, so one
-    // compare against the last threshold decides all eight.  False (nothing
-    // changed) if a lane would need a codeword inside the group or decodes a
-    // 1.  An all-zero codeblock (33 planes, :1155) is decoded entirely here.
+    // compare against the last threshold decides all eight (zero_run).  The
+    // lanes of a codeblock then use up their codewords at the same symbol as a
+    // rule, and the next ones, in lane order, are read ahead and tried for the
+    // rest of the eight.  False, with at most the first step's reservation
+    // made, if a lane decodes a 1 or the lanes differ.  An all-zero codeblock
+    // (33 planes, :1155) is decoded entirely here: about 190 -> 44 us, 2
+    // passes, against groups that a spent codeword ended.
     BPC_FI bool flat_rows(uint32_t P, bool act) {
-        uint32_t sz = E - L, prev = 0;
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            prev = sz;
-            sz = (sz * P) >> 7;
-        }
+        ring_ensure<2>();
+        const bool need = act && L == E;
+        const uint32_t ball = w.ballot(need);
+        if (ball) reserve(need, ball);
         // (probabilities are below 128 in any real table; with others E - L can grow)
-        const bool stop = act && !(P < 128u && E >= L && prev != 0u && cw < L + sz);
-        if (w.any(stop)) return false;
-        if (act) E = L + sz;
+        bool ok = P < 128u && E >= L;
+        uint32_t sz = E - L, prev;
+        zero_run(sz, prev, P);
+        if (!w.any(act && !(ok && prev != 0u && cw < L + sz))) {
+            if (act) E = L + sz;
+            return true;
+        }
+        const int n = zero_count(E - L, P);
+        const uint32_t cw2 = ring[pos + (uint32_t)gl];
+        uint32_t sz2 = 0xFFFFu;
+        bool full = true;
+#pragma unroll
+        for (int k = 1; k < 8; k++) {
+            if (k < n) continue;
+            full = full && sz2 != 0u;
+            sz2 = (sz2 * P) >> 7;
+        }
+        const bool same = n == (int)w.shfl_idx((uint32_t)n, lane & ~(G::NL - 1));
+        ok = ok && same && n < 8 && cw < L && full && cw2 < 1u + sz2;
+        if (w.any(act && !ok)) return false;
+        if (act) {
+            cw = cw2;
+            L = 1u;
+            E = 1u + sz2;
+            pos += (uint32_t)G::NL;
+        }
         return true;
     }
 
@@ -225,12 +290,19 @@ struct Coder<PASSES, CBS, false, W, LAT> {
                 if (flat_rows(P0, act)) continue;
             }
             uint32_t lo = (cur << 8) | last, hi = (cur >> 24) | (nxt << 8), out = 0u;
+            [[maybe_unused]] uint32_t cx = lo;
             uint32_t k8 = PASSES == 3 && PK == PK_CP ? (uint32_t)vis[q * 32] << 9 : 0u;
 #pragma unroll 1
             for (int r = 0; r < 4; r++) {
                 ring_ensure<4>();  // two steps of up to two calls
-                step<PK, 0>(lo, k8, act);
-                step<PK, 1>(lo, k8, act);
+                if constexpr (LAT > 0) {
+                    step_lat<PK, 0>(lo, cx, k8, act);
+                    step_lat<PK, 1>(lo, cx, k8, act);
+                    cx = funnel_r(cx, hi, 8);
+                } else {
+                    step<PK, 0>(lo, k8, act);
+                    step<PK, 1>(lo, k8, act);
+                }
                 lo = funnel_r(lo, hi, 8);
                 hi >>= 8;
                 out = (out >> 8) | (lo << 24);
@@ -272,7 +344,7 @@ struct Coder<PASSES, CBS, false, W, LAT> {
                 const uint32_t bit = u & (0u - u);
                 u ^= bit;
                 ring_ensure<1>();
-                if (ac_dec((R & bit) != 0u, P)) bits |= bit;
+                if (ac_dec<(LAT > 0)>((R & bit) != 0u, P)) bits |= bit;
             }
             planes[b][q] = bits;
         }

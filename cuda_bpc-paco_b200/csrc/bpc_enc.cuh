@@ -436,37 +436,54 @@ struct Coder<PASSES, CBS, true, W, LAT> {
     // read 0 or are never coded here).  Magnitudes out of range (MSB 28..31,
     // flagged) code the same way from their plane down.  All lanes code the
     // same positions, so the warp goes in lockstep, as the decoder does, eight
-    // zeros at a time while no lane needs a codeword.
+    // zeros at a time: the lanes' codewords end at the same symbol as a rule
+    // (they differ in a codeblock that straddles subbands).  139 -> 109 us
+    // for four of them against groups that a spent codeword ended.
+    BPC_FI void zero_reserve(bool need) {
+        const uint32_t ball = w.ballot(need) & gmask;
+        if (need) {
+            store_open();
+            open_slot = (int)(1u + cnt + (uint32_t)popc32(ball & ltmask));
+            L = 1u;
+            E = 0x10000u;
+        }
+        cnt += (uint32_t)popc32(ball);
+    }
     BPC_FI void zero_block(bool flat) {
 #pragma unroll 1
         for (int b = 32; b >= 0; b--) {
             const bool act = flat && b <= msb;
             const uint32_t P = tab[(PASSES == 3 ? p.cp_off : 0) + p.a_sig + (g + b) * 9];
             const bool one = PASSES == 3 && b == 29;
+            // (a probability of 128 or more lets E - L grow)
+            const bool runs = !one && P < 128u;
 #pragma unroll 1
             for (int t = 0; t < 2 * CBS; t += 8) {
-                uint32_t sz = E - L, prev = 0;
-#pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    prev = sz;
-                    sz = (sz * P) >> 7;
-                }
-                // (a probability of 128 or more lets E - L grow)
-                if (!w.any(act && (one || prev == 0u || P >= 128u))) {
+                zero_reserve(act && L == E);
+                uint32_t sz = E - L, prev;
+                zero_run(sz, prev, P);
+                if (!w.any(act && !(runs && prev != 0u))) {
                     if (act) E = L + sz;
+                    continue;
+                }
+                const int n = zero_count(E - L, P);
+                uint32_t sz2 = 0xFFFFu;
+                bool full = true;
+#pragma unroll
+                for (int k = 1; k < 8; k++) {
+                    if (k < n) continue;
+                    full = full && sz2 != 0u;
+                    sz2 = (sz2 * P) >> 7;
+                }
+                const bool same = n == (int)w.shfl_idx((uint32_t)n, lane & ~(G::NL - 1));
+                if (!w.any(act && !(runs && n < 8 && same && full))) {
+                    zero_reserve(act);
+                    if (act) E = L + sz2;
                     continue;
                 }
 #pragma unroll 1
                 for (int k = 0; k < 8; k++) {
-                    const bool need = act && L == E;
-                    const uint32_t ball = w.ballot(need) & gmask;
-                    if (need) {
-                        store_open();
-                        open_slot = (int)(1u + cnt + (uint32_t)popc32(ball & ltmask));
-                        L = 1u;
-                        E = 0x10000u;
-                    }
-                    cnt += (uint32_t)popc32(ball);
+                    zero_reserve(act && L == E);
                     const uint32_t thr = L + (((E - L) * P) >> 7);
                     if (act && one) L = thr + 1u;
                     if (act && !one) E = thr;

@@ -51,6 +51,28 @@ def test_damaged_zero_codeblocks(emu, oracle_mod, passes, cb):  # noqa: F811
         assert st == int(np.bitwise_or.reduce(wst))
 
 
+@pytest.mark.parametrize("passes", [2, 3])
+@pytest.mark.parametrize("cb", [64, 32])
+def test_zero_codeblocks(emu, oracle_mod, passes, cb):  # noqa: F811
+    """All-zero codeblocks, inside one subband (all lanes' codewords end at the
+    same symbol) and straddling several; with random probabilities the ends
+    fall on every symbol of the eight-symbol groups."""
+    z = np.zeros((cb, 2 * cb), np.int32)
+    rng = np.random.default_rng(passes + cb)
+    for levels in (1, 5):
+        lut0 = oracle_mod.load_luts(lut_folder(passes), passes, levels)
+        for lut in (lut0, rng.integers(1, 128, size=lut0.size).astype(np.int32),
+                    rng.integers(100, 128, size=lut0.size).astype(np.int32)):
+            want, wst = oracle_mod.encode(z, lut, passes, levels, cb, with_status=True)
+            got, st = run(emu, 1, z, z.shape, lut, passes, levels, cb)
+            np.testing.assert_array_equal(got, want)
+            assert st == int(np.bitwise_or.reduce(wst))
+            wdec = oracle_mod.decode(want, z.shape, lut, passes, levels, cb)
+            for kind in (0, 2):
+                dec, _ = run(emu, 0, want, z.shape, lut, passes, levels, cb, kind=kind)
+                np.testing.assert_array_equal(dec.reshape(z.shape), wdec)
+
+
 @pytest.mark.parametrize("passes,cb", [(2, 64), (3, 32)])
 @pytest.mark.parametrize("lo,hi", [(0, 3), (126, 131), (200, 256)])
 def test_unusual_probabilities(emu, oracle_mod, passes, cb, lo, hi):  # noqa: F811
