@@ -11,14 +11,14 @@
 // codes which codeblock, never a stream word or a coefficient.
 //
 // Expected work of a work unit (the NG codeblocks one warp codes):
-//   decoder: the slot words in use (MSB word + codewords), found by a binary
-//            search for the first -1 of the fill (codewords are 0..0xFFFF;
-//            on a damaged slot the search still ends inside it, and only the
-//            order is affected), plus kPlaneWords per bitplane decoded;
-//   encoder: the bitplanes coded, MSB + 1 (33 for an all-zero codeblock),
-//            from one read of the coefficients.
-// One CTA then counting-sorts the units by cost, descending (warp-aggregated
-// shared-memory atomics; units of equal cost in any order).
+//   decoder: the slot words in use (MSB word + codewords), found by a search
+//            for the first -1 of the fill (codewords are 0..0xFFFF; on a
+//            damaged slot the search still ends inside it, and only the order
+//            is affected), plus kPlaneWords per bitplane decoded;
+//   encoder: the bitplanes coded, MSB + 1 (33 for an all-zero codeblock), from
+//            all or, in a large image, every eighth row of the coefficients.
+// The units are then counting-sorted by cost, descending (shared-memory atomics;
+// units of equal cost in any order).
 //
 // An isolated decode (launch_code) takes the first units of the order for its
 // heavy launch and hands the rest out from a queue counter that follows the
@@ -43,33 +43,50 @@ constexpr int kBuckets = 1024;  // = threads of the sorting CTA
 // ms; with 128: 0.597 ms; with 64: 0.601 ms).
 constexpr uint32_t kPlaneWords = 128, kPlaneWordsIso = 256;
 
+// Eight lanes per unit.  The first -1 is found eight probes at a time (four
+// dependent loads) instead of by bisection, whose twelve were 9 us before a
+// 4096x4096 decode could start; 32 probes at a time touch three times the
+// sectors (16384x16384: 47 us).
 template <int CBS>
 __global__ void k_cost_dec(const int32_t *in, int ncb, uint32_t plane_words, uint32_t *key) {
     using G = Geo<CBS>;
     const int units = (ncb + G::NG - 1) / G::NG;
-    for (int u = (int)(blockIdx.x * blockDim.x + threadIdx.x); u < units; u += (int)(gridDim.x * blockDim.x)) {
+    const int lane = (int)(threadIdx.x & 31u), grp = lane >> 3, l8 = lane & 7;
+    const int wstride = (int)(gridDim.x * blockDim.x) >> 5;
+    for (int u4 = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; 4 * u4 < units; u4 += wstride) {
+        const int u = 4 * u4 + grp;
         uint32_t cost = 0;
+#pragma unroll
         for (int k = 0; k < G::NG; k++) {
             const int cb = u * G::NG + k;
-            if (cb >= ncb) break;
-            const int32_t *slot = in + (size_t)cb * (size_t)G::CAP;
-            int lo = 1, hi = G::CAP;  // first index >= 1 holding -1 (CAP if none)
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (__ldg(slot + mid) == -1)
-                    hi = mid;
-                else
-                    lo = mid + 1;
-            }
+            const bool ok = cb < ncb;
+            const int32_t *slot = in + (size_t)(ok ? cb : 0) * (size_t)G::CAP;
             const int m = __ldg(slot);  // MSB word: planes decoded
+            // words [lo, lo + 8 step) hold the first -1, if there is one; a
+            // probe that reads a codeword moves lo behind it
+            int lo = 0;
+#pragma unroll
+            for (int step = G::CAP / 8; step > 0; step = step > 1 && step < 8 ? 1 : step / 8) {
+                const int i = lo + (l8 + 1) * step - 1;
+                const bool used = i < G::CAP && __ldg(slot + (i < G::CAP ? i : 0)) != -1;
+                const unsigned b = (__ballot_sync(0xffffffffu, used) >> (8 * grp)) & 0xFFu;
+                lo += step * (__ffs((int)~b) - 1);
+            }
             const uint32_t planes = m == 32 ? 33u : (m >= 0 && m <= 27 ? (uint32_t)m + 1u : 0u);
-            cost += (uint32_t)lo + plane_words * planes;
+            if (ok) cost += (uint32_t)(lo < 1 ? 1 : lo) + plane_words * planes;
         }
-        key[u] = cost;
+        if (l8 == 0 && u < units) key[u] = cost;
     }
 }
 
-template <int CBS>
+// The bitplanes of a codeblock from every ROWS-th of its rows.  Every eighth is
+// enough to order the codeblocks of a large image (16384x16384: reading it
+// whole took 150 us; the encode 3.94 -> 3.86 ms).  Up to kWholeCoeffs the whole
+// image is read: what the L2 keeps of it the coder need not fetch again
+// (2-pass encodes, whole / every eighth row: 6144x6144 0.395 / 0.425 ms, 8192x8192
+// 0.677 / 0.703, 12288x12288 1.557 / 1.552).
+constexpr long long kWholeCoeffs = 72ll << 20;
+template <int CBS, int ROWS>
 __global__ void k_cost_enc(const int32_t *in, int X, int ncbx, int ncb, uint32_t *key) {
     using G = Geo<CBS>;
     const int units = (ncb + G::NG - 1) / G::NG;
@@ -81,7 +98,8 @@ __global__ void k_cost_enc(const int32_t *in, int X, int ncbx, int ncb, uint32_t
         if (cb < ncb) {
             const int cbx = cb % ncbx, cby = cb / ncbx;
             const int32_t *src = in + (size_t)cby * CBS * (size_t)X + (size_t)cbx * CBS + 2 * gl;
-            for (int i = 0; i < CBS; i++) {
+#pragma unroll 8
+            for (int i = ROWS / 2; i < CBS; i += ROWS) {
                 const int2 v = __ldg(reinterpret_cast<const int2 *>(src + (size_t)i * (size_t)X));
                 mx |= (v.x < 0 ? 0u - (uint32_t)v.x : (uint32_t)v.x) | (v.y < 0 ? 0u - (uint32_t)v.y : (uint32_t)v.y);
             }
@@ -99,24 +117,55 @@ __device__ __forceinline__ int cost_bin(uint32_t cost, int shift) {
     return kBuckets - 1 - (int)(b > (uint32_t)(kBuckets - 1) ? (uint32_t)(kBuckets - 1) : b);
 }
 
+// Counting sort.  Every CTA counts the bins of all units, and apart from that
+// those of the units before its own share, and so knows where its share goes
+// without talking to the others; the loads of several rounds are in flight
+// together.  (One CTA, one load at a time: 58 us for the encoder's 65536 units,
+// 74 for the decoder's, 9 for a decoder's 4096.)
+//
+// COARSE (encoder, a few dozen different costs): a warp's units of equal cost
+// claim their places together and stay in raster order.  Scattered one by one
+// the same costs make a 6144x6144 encode 5 % slower (neighbouring codeblocks
+// then run far apart).  The decoder's costs are nearly all different: it takes
+// places one by one.
+constexpr int kOrderAhead = 8, kOrderShare = 4 * kBuckets;
+template <bool COARSE>
 __global__ void __launch_bounds__(kBuckets) k_order(const uint32_t *key, int units, int shift, int ng, int *order,
                                                     int *ctr) {
-    __shared__ uint32_t next[kBuckets];
+    __shared__ uint32_t all[kBuckets], next[kBuckets];
     __shared__ uint32_t wsum[kBuckets / 32];
     const int tid = (int)threadIdx.x, lane = tid & 31;
-    if (tid == 0 && ctr) *ctr = 0;  // the isolated decode's queue counter
-    next[tid] = 0;
+    if (tid == 0 && blockIdx.x == 0 && ctr) *ctr = 0;  // the isolated decode's queue counter
+    all[tid] = next[tid] = 0;
     __syncthreads();
-    // whole warps step through the units together (full-mask warp calls)
-    for (int u0 = tid - lane; u0 < units; u0 += kBuckets) {
-        const int u = u0 + lane;
-        const int bin = u < units ? cost_bin(key[u], shift) : -1;
-        const unsigned peers = __match_any_sync(0xffffffffu, bin);
-        if (bin >= 0 && lane == __ffs(peers) - 1) atomicAdd(&next[bin], (uint32_t)__popc(peers));
+    const int s0 = (int)blockIdx.x * kOrderShare, s1 = s0 + kOrderShare < units ? s0 + kOrderShare : units;
+    // whole warps step through the units together (full-mask warp calls); s0
+    // is a multiple of the warp's 32, so a warp's units lie on one side of it
+    for (int u0 = tid - lane; u0 < units; u0 += kBuckets * kOrderAhead) {
+        int bin[kOrderAhead];
+#pragma unroll
+        for (int k = 0; k < kOrderAhead; k++) {
+            const int u = u0 + k * kBuckets + lane;
+            bin[k] = u < units ? cost_bin(__ldg(key + u), shift) : -1;
+        }
+#pragma unroll
+        for (int k = 0; k < kOrderAhead; k++) {
+            uint32_t n = 1u;
+            bool mine = bin[k] >= 0;
+            if constexpr (COARSE) {
+                const unsigned peers = __match_any_sync(0xffffffffu, bin[k]);
+                n = (uint32_t)__popc(peers);
+                mine = mine && lane == __ffs((int)peers) - 1;
+            }
+            if (mine) {
+                atomicAdd(&all[bin[k]], n);
+                if (u0 + k * kBuckets < s0) atomicAdd(&next[bin[k]], n);
+            }
+        }
     }
     __syncthreads();
     // exclusive scan of the bin counts
-    const uint32_t v = next[tid];
+    const uint32_t v = all[tid];
     uint32_t x = v;
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
@@ -133,18 +182,22 @@ __global__ void __launch_bounds__(kBuckets) k_order(const uint32_t *key, int uni
         wsum[tid] = y;
     }
     __syncthreads();
-    next[tid] = x - v + (tid >= 32 ? wsum[(tid >> 5) - 1] : 0u);
+    next[tid] += x - v + (tid >= 32 ? wsum[(tid >> 5) - 1] : 0u);
     __syncthreads();
-    for (int u0 = tid - lane; u0 < units; u0 += kBuckets) {
-        const int u = u0 + lane;
-        const int bin = u < units ? cost_bin(key[u], shift) : -1;
-        const unsigned peers = __match_any_sync(0xffffffffu, bin);
-        const int leader = __ffs(peers) - 1;
-        uint32_t base = 0;
-        if (bin >= 0 && lane == leader) base = atomicAdd(&next[bin], (uint32_t)__popc(peers));
-        base = __shfl_sync(0xffffffffu, base, leader);
-        const uint32_t rank = (uint32_t)__popc(peers & ((1u << lane) - 1u));
-        if (bin >= 0) order[base + rank] = u * ng;
+    for (int r0 = s0; r0 < s1; r0 += kBuckets) {  // the whole CTA, round by round
+        const int u = r0 + tid;
+        const int bin = u < s1 ? cost_bin(__ldg(key + u), shift) : -1;
+        if constexpr (COARSE) {
+            const unsigned peers = __match_any_sync(0xffffffffu, bin);
+            const int leader = __ffs((int)peers) - 1;
+            uint32_t base = 0;
+            if (bin >= 0 && lane == leader) base = atomicAdd(&next[bin], (uint32_t)__popc(peers));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            if (bin >= 0) order[base + (uint32_t)__popc(peers & ((1u << lane) - 1u))] = u * ng;
+            __syncthreads();  // the rounds in order, too
+        } else if (bin >= 0) {
+            order[atomicAdd(&next[bin], 1u)] = u * ng;
+        }
     }
 }
 
@@ -192,9 +245,12 @@ cudaError_t plan_t(bool enc, Params &p, int *sched, cudaStream_t st, bool iso) {
     const uint32_t plane_words = iso ? kPlaneWordsIso : kPlaneWords;
     if (enc) {  // one warp per unit, grid-stride
         const int grid = (units + 7) / 8 < 4096 ? (units + 7) / 8 : 4096;
-        k_cost_enc<CBS><<<grid, 256, 0, st>>>(p.in, p.X, p.ncbx, p.ncb, key);
-    } else {  // one thread per unit, grid-stride
-        const int grid = (units + 255) / 256 < 1024 ? (units + 255) / 256 : 1024;
+        if ((long long)p.X * p.Y <= kWholeCoeffs)
+            k_cost_enc<CBS, 1><<<grid, 256, 0, st>>>(p.in, p.X, p.ncbx, p.ncb, key);
+        else
+            k_cost_enc<CBS, 8><<<grid, 256, 0, st>>>(p.in, p.X, p.ncbx, p.ncb, key);
+    } else {
+        const int grid = (units + 31) / 32 < 4096 ? (units + 31) / 32 : 4096;
         k_cost_dec<CBS><<<grid, 256, 0, st>>>(p.in, p.ncb, plane_words, key);
     }
     // bins of 2^shift cost units: decoder costs reach NG * (CAP + 33 * plane
@@ -205,7 +261,11 @@ cudaError_t plan_t(bool enc, Params &p, int *sched, cudaStream_t st, bool iso) {
         while ((mx >> shift) > kBuckets - 1) shift++;
     }
     int *ctr = iso ? sched + 2 * units : nullptr;
-    k_order<<<1, kBuckets, 0, st>>>(key, units, shift, G::NG, sched, ctr);
+    const int ctas = (units + kOrderShare - 1) / kOrderShare;
+    if (enc)
+        k_order<true><<<ctas, kBuckets, 0, st>>>(key, units, shift, G::NG, sched, ctr);
+    else
+        k_order<false><<<ctas, kBuckets, 0, st>>>(key, units, shift, G::NG, sched, ctr);
     p.order = sched;
     p.ctr = ctr;
     return cudaGetLastError();
