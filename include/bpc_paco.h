@@ -167,7 +167,8 @@ int bpc_batch_encode(void *batch, const int *const *d_coeffs, int *d_compact, lo
 int bpc_batch_decode(void *batch, const int *d_compact, const long long *d_offsets, int *const *d_coeffs,
                      int *d_status, void *stream);
 /* Schedule: CTAs per SM for the encoder (1..4) and decoder (1..7), codeblocks
- * per work item, CUDA graph on/off.  bpc_batch_tune times the candidates on the
+ * per work item (at most: a batch too small to give every warp many items uses
+ * shorter ones), CUDA graph on/off.  bpc_batch_tune times the candidates on the
  * given buffers and keeps the fastest. */
 int bpc_batch_set_schedule(void *batch, int ctas_per_sm_enc, int ctas_per_sm_dec, int cbs_per_item, int use_graph);
 int bpc_batch_get_schedule(const void *batch, int *ctas_per_sm_enc, int *ctas_per_sm_dec, int *cbs_per_item,
