@@ -289,38 +289,35 @@ constexpr int kEvKeys = 1, kEvVals = 512;
 // move to its first half through memory again: they are in L2 or L1, and this
 // runs once per 256 codewords.)  Kept out of line: inlined into every decoder
 // step body it would crowd the instruction cache.
+// All loads are issued before the first word is stored, so a refill waits for
+// memory once and not four times (a codeblock decoded alone refills up to eight
+// times: 186 -> 178 us, 2 passes).
 template <int CBS>
 BPC_NOINLINE void ring_fill(uint32_t *ring, const int32_t *slot_in, uint32_t in_cap, bool compact, uint32_t first,
                             int gl) {
     using G = Geo<CBS>;
     constexpr int per = G::RING / G::NL;  // 16, a multiple of 4
+    uint32_t v[per];
+#pragma unroll
     for (int q = 0; q < per; q += 4) {
-        const uint32_t r = (uint32_t)(q * G::NL + 4 * gl), k = first + r;
-        uint32_t v0, v1, v2, v3;
+        const uint32_t k = first + (uint32_t)(q * G::NL + 4 * gl);
         if (k + 3 < in_cap && !compact) {
 #if defined(__CUDA_ARCH__)
-            const int4 v = *reinterpret_cast<const int4 *>(slot_in + k);
-            v0 = (uint32_t)v.x;
-            v1 = (uint32_t)v.y;
-            v2 = (uint32_t)v.z;
-            v3 = (uint32_t)v.w;
+            const int4 t = __ldg(reinterpret_cast<const int4 *>(slot_in + k));
+            v[q] = (uint32_t)t.x;
+            v[q + 1] = (uint32_t)t.y;
+            v[q + 2] = (uint32_t)t.z;
+            v[q + 3] = (uint32_t)t.w;
 #else
-            v0 = (uint32_t)slot_in[k];
-            v1 = (uint32_t)slot_in[k + 1];
-            v2 = (uint32_t)slot_in[k + 2];
-            v3 = (uint32_t)slot_in[k + 3];
+            for (int i = 0; i < 4; i++) v[q + i] = (uint32_t)slot_in[k + i];
 #endif
         } else {  // slot end, or the compact container (no 16-byte alignment)
-            v0 = k + 0 < in_cap ? (uint32_t)slot_in[k + 0] : 0xFFFFFFFFu;
-            v1 = k + 1 < in_cap ? (uint32_t)slot_in[k + 1] : 0xFFFFFFFFu;
-            v2 = k + 2 < in_cap ? (uint32_t)slot_in[k + 2] : 0xFFFFFFFFu;
-            v3 = k + 3 < in_cap ? (uint32_t)slot_in[k + 3] : 0xFFFFFFFFu;
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[q + i] = k + i < in_cap ? (uint32_t)slot_in[k + i] : 0xFFFFFFFFu;
         }
-        ring[r] = v0;
-        ring[r + 1] = v1;
-        ring[r + 2] = v2;
-        ring[r + 3] = v3;
     }
+#pragma unroll
+    for (int q = 0; q < per; q++) ring[(q & ~3) * G::NL + 4 * gl + (q & 3)] = v[q];
 }
 
 template <class W>
