@@ -133,14 +133,14 @@ def launches_per_call(X, Y, cb, enc, dev):
     """Kernels one work-ordered call launches: the coder, plus the cost and
     sort kernels when the image spans more than two waves of resident warps
     (4 warps x 5 encoder / 7 decoder CTAs per SM); a decode of 64x64
-    codeblocks between half a wave and two waves is sorted too and isolated
+    codeblocks between nine tenths of a wave and two waves is sorted too and isolated
     (heavy launch + bulk launch)."""
     import torch
     units = (X // cb) * (Y // cb) // (1 if cb == 64 else 2)
     resident = torch.cuda.get_device_properties(dev).multi_processor_count * 4 * (5 if enc else 7)
     if units >= 2 * resident:
         return 3
-    if not enc and cb == 64 and 2 * units > resident and units > 4 * 6 * 4:
+    if not enc and cb == 64 and 10 * units > 9 * resident and units > 4 * 6 * 4:
         return 4
     return 1
 

@@ -82,7 +82,7 @@ __device__ __forceinline__ void stage_lut(const Params &p, uint8_t *tab) {
     if (bad && p.status) atomicOr(p.status, ST_LUT_RANGE);
 }
 
-// WARPS codeblock warps per CTA: kWarps, or 1 for decodes of at most half a wave
+// WARPS codeblock warps per CTA: kWarps, or 1 for decodes of at most one wave
 // (their heaviest codeblocks then land on different SMs, see launch_t); the
 // register budget stays that of kMinCtas x kWarps resident warps per SM
 template <int PASSES, int CBS, bool ENC, int WARPS = kWarps, int LAT = 0>
@@ -272,18 +272,21 @@ static cudaError_t launch_t(const Params &p, int grid, cudaStream_t st, bool lat
         return launch_w<PASSES, CBS, ENC, kWarps, 0>(p, grid, warps_needed, st);
     } else {
         const long long resident = resident_warps(ENC, -1);
-        // A decode of at most half a wave of resident warps runs one warp per
-        // CTA (consecutive CTAs go to different SMs, so its heaviest codeblocks,
-        // the coarse subbands, neighbours in raster order, do not share an SM's
-        // instruction cache and shared-memory pipes; a 2048x2048 decode: 0.375
-        // -> 0.358 ms) and the latency form of the step.  Fuller decodes keep
-        // 4-warp CTAs and the form with fewer instructions, which measured
-        // faster there.  A work-ordered whole image the planner marked for
-        // isolation (p.ctr set) runs its heaviest codeblocks on SMs of their own.
+        // A work-ordered whole image the planner marked for isolation (p.ctr
+        // set) runs its heaviest codeblocks on SMs of their own.  Other decodes
+        // of at most one wave of resident warps run one warp per CTA, in the
+        // latency form of the step: consecutive CTAs go to different SMs, so
+        // the heaviest codeblocks (the coarse subbands, neighbours in raster
+        // order) do not share one, no SM gets a whole CTA more than another,
+        // and the warps that shared memory leaves waiting start as others end
+        // (3-pass decodes, 4-warp / one-warp CTAs: 2944x2944 0.387 / 0.318 ms,
+        // 3456x3456 0.404 / 0.334, 4096x4096 0.394 / 0.376).  Fuller ones keep
+        // 4-warp CTAs and the form with fewer instructions (5760x5760 0.550 /
+        // 0.568).
         if constexpr (CBS == 64) {
             if (lat && grid <= 0 && p.order && p.ctr) return launch_iso<PASSES, CBS>(p, st);
         }
-        if (lat && grid <= 0 && 2LL * warps_needed <= resident)
+        if (lat && grid <= 0 && !p.order && warps_needed <= resident)
             return launch_w<PASSES, CBS, ENC, 1, 1>(p, grid, warps_needed, st);
         return launch_w<PASSES, CBS, ENC, kWarps, 0>(p, grid, warps_needed, st);
     }

@@ -50,7 +50,7 @@ int code_device(bool enc, const int *in, int *out, int X, int Y, const int *d_lu
 // sched_ints(ncb, cbs) ints, queue the kernels that sort the image's work
 // units by expected cost, heaviest first, and set p.order.  Images of more than
 // two waves are sorted for a balanced last wave; decodes of 64x64 codeblocks
-// between half a wave and two waves are sorted for an isolated launch
+// between nine tenths of a wave and two waves are sorted for an isolated launch
 // (launch_code) when `isolate` allows it, which also sets p.ctr to the bulk
 // launch's queue counter in the scratch.  Other images keep raster order
 // (p.order and p.ctr stay null).

@@ -292,13 +292,15 @@ cudaError_t plan_order(bool enc, int cbs, Params &p, int *sched, cudaStream_t st
     if (!sched || p.offsets || p.cb_begin != 0 || p.cb_end != p.ncb) return cudaSuccess;
     if (order_pays(enc, p.ncb, cbs))
         return cbs == 64 ? plan_t<64>(enc, p, sched, st, false) : plan_t<32>(enc, p, sched, st, false);
-    // isolated decode: 64x64 codeblocks, more than half a wave (smaller decodes
-    // already spread one warp per CTA), more than the heavy launch's share, and
-    // a device with SMs to spare for it
+    // isolated decode: 64x64 codeblocks, more than nine tenths of a wave (below
+    // that one-warp CTAs in raster order are faster: 3840x3840, 0.87 of a wave,
+    // isolated / one-warp 0.362 / 0.352 ms in 3 passes, 0.251 / 0.246 in 2;
+    // 4096x4096, 0.99, 0.345 / 0.376 and 0.251 / 0.248), more than the heavy
+    // launch's share, and a device with SMs to spare for it
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return cudaSuccess;
     const long long res = resident_warps(false, dev);
-    if (isolate && !enc && cbs == 64 && 2LL * p.ncb > res && p.ncb > 4 * kIsoCtas * kWarps &&
+    if (isolate && !enc && cbs == 64 && 10LL * p.ncb > 9 * res && p.ncb > 4 * kIsoCtas * kWarps &&
         sm_count(dev) > 4 * kIsoCtas && shared_optin(dev) > 0)
         return plan_t<64>(enc, p, sched, st, true);
     return cudaSuccess;

@@ -129,12 +129,13 @@ int bpc_decode_device(const int *d_stream, int *d_coeffs, int X, int Y, const in
                       int levels, int cb_size, int *d_status, int *d_counts, int grid, void *stream);
 
 /* The same calls with a work order: for images of more than two waves of
- * warps (above about 4,700 codeblocks for the encoder, 8,300 for the decoder
+ * warps (above about 5,900 codeblocks for the encoder, 8,300 for the decoder
  * on a 148-SM B200) the call first sorts the codeblocks by expected work,
  * heaviest first (decoder: slot words in use and bitplanes; encoder: bitplanes
- * coded, from one read of the coefficients), so that the warps of a CTA finish
- * together and the last wave is short.  A decode of 64x64 codeblocks between
- * half a wave and two waves (about 2,100 to 8,300 codeblocks, e.g. 4096x4096)
+ * coded, from a read of the coefficients, every eighth row of a large image), so
+ * that the warps of a CTA finish together and the last wave is short.  A decode
+ * of 64x64 codeblocks between nine tenths of a wave and two waves (about 3,700
+ * to 8,300 codeblocks, e.g. 4096x4096)
  * is sorted the same way and then isolated: its 24 heaviest codeblocks run on
  * six SMs of their own, the rest on the other SMs as a programmatic dependent
  * launch that starts once those are resident.  Outputs are identical to the
