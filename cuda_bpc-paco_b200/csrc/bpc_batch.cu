@@ -26,6 +26,7 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <map>
+#include <tuple>
 #include <vector>
 
 #include "../../include/bpc_paco.h"
@@ -572,7 +573,7 @@ void free_batch(Batch *b) {
 int create(Batch &b, int n, const int *X, const int *Y, const int *levels, const int *passes, const int *cbsz,
            const int *const *d_luts, const int *lut_n) {
     b.n = n;
-    std::map<std::pair<const int *, int>, uint8_t *> tab_cache;
+    std::map<std::tuple<const int *, int, int>, uint8_t *> tab_cache;
     for (int i = 0; i < n; i++) {
         if ((passes[i] != 2 && passes[i] != 3) || (cbsz[i] != 64 && cbsz[i] != 32) || levels[i] < 1 ||
             levels[i] > 16 || X[i] <= 0 || Y[i] <= 0 || X[i] % cbsz[i] || Y[i] % cbsz[i] || !d_luts[i] ||
@@ -587,7 +588,7 @@ int create(Batch &b, int n, const int *X, const int *Y, const int *levels, const
         b.ncb += (long long)(X[i] / cbsz[i]) * (Y[i] / cbsz[i]);
         b.words += (long long)X[i] * Y[i];
         const int tab_n = lut_offsets(levels[i], passes[i], lut_n[i]).tab_n;
-        auto key = std::make_pair(d_luts[i], tab_n);
+        auto key = std::make_tuple(d_luts[i], lut_n[i], tab_n);
         auto it = tab_cache.find(key);
         if (it == tab_cache.end()) {
             uint8_t *t = nullptr;

@@ -121,11 +121,14 @@ struct Params {
 };
 
 // LUT offsets the reference kernel uses (Initialize_LUT_pointers :228-250 with
-// LUT_N_BITPLANES = 15, and the CP offset :988-989).
+// LUT_N_BITPLANES = 15, and the CP offset :988-989).  tab_n, the bytes of table
+// a kernel keeps, depends on the mode alone (at most 19,920, at 16 levels and 3
+// passes): entries of a longer LUT that the coder cannot index are range-checked
+// and not kept, so the shared memory of a launch does not grow with the LUT.
 struct LutOffsets {
     int a_sig, a_sign, cp_off, tab_n;
 };
-inline LutOffsets lut_offsets(int levels, int passes, int lut_n) {
+inline LutOffsets lut_offsets(int levels, int passes, int /*lut_n*/) {
     LutOffsets o;
     const int ref_n = 3 * 15 * 1 * levels + 15 * 1;
     const int sig_n = 3 * 15 * 9 * levels + 15 * 9;
@@ -143,9 +146,7 @@ inline LutOffsets lut_offsets(int levels, int passes, int lut_n) {
     }
     mx = mx > s1 ? mx : s1;
     mx = mx > s2 ? mx : s2;
-    int n = mx + 1;
-    if (n < lut_n) n = lut_n;
-    o.tab_n = (n + 15) & ~15;
+    o.tab_n = (mx + 1 + 15) & ~15;
     return o;
 }
 

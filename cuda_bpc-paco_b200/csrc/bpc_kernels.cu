@@ -48,8 +48,8 @@ struct GpuWarp {
     __device__ __forceinline__ void atomic_or(int *p, int v) { atomicOr(p, v); }
 };
 
-// The LUT as bytes in shared memory, zero-padded to tab_n; entries outside
-// 0..255 are flagged and read as 0.  Four entries per load and several loads in
+// The LUT's first tab_n entries as bytes in shared memory (zeros where it is
+// shorter); entries outside 0..255, also past tab_n, are flagged and read as 0.  Four entries per load and several loads in
 // flight per thread: a CTA starts with this, and one load after another it took
 // 10-15 us of a small image's time (one-warp CTAs, 6480 entries).
 __device__ __forceinline__ void stage_lut(const Params &p, uint8_t *tab) {
@@ -67,17 +67,19 @@ __device__ __forceinline__ void stage_lut(const Params &p, uint8_t *tab) {
             v.z = (unsigned)v.z > 255u ? 0 : v.z;
             v.w = (unsigned)v.w > 255u ? 0 : v.w;
         }
-        reinterpret_cast<uchar4 *>(tab)[k] =
-            make_uchar4((unsigned char)v.x, (unsigned char)v.y, (unsigned char)v.z, (unsigned char)v.w);
+        if (4 * k < p.tab_n)  // tab_n is a multiple of 16
+            reinterpret_cast<uchar4 *>(tab)[k] =
+                make_uchar4((unsigned char)v.x, (unsigned char)v.y, (unsigned char)v.z, (unsigned char)v.w);
     }
+    const int end = p.lut_n > p.tab_n ? p.lut_n : p.tab_n;
 #pragma unroll 4
-    for (int k = 4 * n4 + (int)threadIdx.x; k < p.tab_n; k += (int)blockDim.x) {
+    for (int k = 4 * n4 + (int)threadIdx.x; k < end; k += (int)blockDim.x) {
         int v = k < p.lut_n ? __ldg(p.lut + k) : 0;
         if (v < 0 || v > 255) {
             bad = 1;
             v = 0;
         }
-        tab[k] = (uint8_t)v;
+        if (k < p.tab_n) tab[k] = (uint8_t)v;
     }
     if (bad && p.status) atomicOr(p.status, ST_LUT_RANGE);
 }
@@ -177,7 +179,7 @@ static size_t smem_bytes(const Params &p) {
     return (size_t)p.tab_n + (size_t)kSignTableBytes + (size_t)WARPS * 4u * (size_t)(ENC ? 512 : G::RING_WORDS);
 }
 
-// The shared memory a launch asks for grows with the LUT's length, and the
+// The shared memory a launch asks for grows with the mode's DWT levels, and the
 // attribute that admits it belongs to the kernel, not to the launch: host
 // threads set it and launch under this lock, so no launch meets a smaller
 // setting another thread made in between.
@@ -220,6 +222,10 @@ static cudaError_t launch_iso(const Params &p, cudaStream_t st) {
     const int optin = shared_optin(dev), sms = sm_count(dev);
     if (optin <= 0 || sms <= kIsoCtas) return cudaErrorInvalidValue;
     const int units = (p.ncb + G::NG - 1) / G::NG;
+    // both launches stage the same table; the heavy one asks for the opt-in
+    // maximum, so whether that is enough is settled before either goes out
+    const size_t sm = smem_bytes<PASSES, CBS, false, kWarps>(p);
+    if (sm > (size_t)optin) return cudaErrorInvalidValue;
     Params ph = p;
     ph.heavy = 1;
     ph.heavy_n = kIsoCtas * kWarps;
@@ -231,7 +237,6 @@ static cudaError_t launch_iso(const Params &p, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     Params pb = ph;
     pb.heavy = 2;
-    const size_t sm = smem_bytes<PASSES, CBS, false, kWarps>(pb);
     e = cudaFuncSetAttribute(k_bpc<PASSES, CBS, false, kWarps, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sm);
     if (e != cudaSuccess) return e;
@@ -294,6 +299,7 @@ static cudaError_t launch_t(const Params &p, int grid, cudaStream_t st, bool lat
 
 cudaError_t launch_code(bool enc, int passes, int cbs, const Params &p, int grid, cudaStream_t st, bool lat) {
     if (p.cb_end <= p.cb_begin) return cudaSuccess;
+    if (p.lut_n > kMaxLut) return cudaErrorInvalidValue;
     if (enc) {
         if (passes == 2)
             return cbs == 64 ? launch_t<2, 64, true>(p, grid, st, lat) : launch_t<2, 32, true>(p, grid, st, lat);

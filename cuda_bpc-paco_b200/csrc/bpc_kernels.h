@@ -30,6 +30,10 @@ constexpr int kMinCtasEnc = ENC_MIN_CTAS;
 constexpr unsigned kEncInAlign = 8, kDecInAlign = 16;
 inline bool aligned_to(const void *p, unsigned a) { return ((uintptr_t)p & (uintptr_t)(a - 1)) == 0; }
 
+// Longest LUT a launch takes (every CTA reads all of it, for the range check).
+// The longest table a mode has, 16 levels and 3 passes, is 19,845 entries.
+constexpr int kMaxLut = 230144;
+
 // Launch the encoder (enc) or decoder over p.ncb codeblocks.  grid <= 0 picks
 // one CTA per kWarps codeblocks; a positive grid runs persistent CTAs that
 // walk the codeblocks grid-stride.  latency_forms lets a decode of a few waves
