@@ -31,10 +31,11 @@
 #include <cstdio>
 
 #include "../../include/bpc_paco.h"
+#include "bpc_dwt_plan.h"
 
 namespace {
 
-constexpr int kThreads = 128;
+constexpr int kThreads = bpc::kDwtThreads;
 constexpr unsigned kFull = 0xffffffffu;
 
 // Vertical pairs per thread.  A strip reads 3 rows above its own again (from L2:
@@ -223,10 +224,30 @@ __global__ void __launch_bounds__(kThreads) k_inv(const int32_t *in, int32_t *ou
 
 // The details of levels 1, 3, ... (and, with whole, the low band of level
 // `levels`) from one raster to the other.  blockIdx.y counts row groups of
-// level 1, then of level 3, and so on.
+// level 1, then of level 3, and so on.  Levels up to vec_level go with 16-byte
+// accesses (dwt_copy_vec_level); WIDE / NARROW: some levels do / do not (both
+// ways in every launch cost 3072x2048 1 us of 43).
 constexpr int kCopyRows = 4;
 template <int V>
-__global__ void __launch_bounds__(kThreads) k_copy_odd(const int32_t *in, int32_t *out, long long stride, int X, int Y, int levels) {
+__device__ __forceinline__ void copy_rows(const int32_t *in, int32_t *out, long long stride, int w, int h, int r0, int c,
+                                          bool whole) {
+    if (c >= w) return;
+    int32_t v[kCopyRows][V];
+    bool on[kCopyRows];
+#pragma unroll
+    for (int k = 0; k < kCopyRows; k++) {
+        const int r = r0 + k;
+        // the low quadrant belongs to the next level, unless this is the last
+        on[k] = r < h && (whole || r >= (h >> 1) || c >= (w >> 1));
+        if (on[k]) load_run<V>(in + (long long)r * stride + c, v[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < kCopyRows; k++)
+        if (on[k]) store_run<V>(out + (long long)(r0 + k) * stride + c, v[k]);
+}
+template <bool WIDE, bool NARROW>
+__global__ void __launch_bounds__(kThreads) k_copy_odd(const int32_t *in, int32_t *out, long long stride, int X, int Y,
+                                                       int levels, int vec_level) {
     after_previous();
     int y = (int)blockIdx.y, l = 1;
     for (; l <= levels; l += 2) {
@@ -234,27 +255,12 @@ __global__ void __launch_bounds__(kThreads) k_copy_odd(const int32_t *in, int32_
         if (y < groups) break;
         y -= groups;
     }
-    const int w = X >> (l - 1), h = Y >> (l - 1);
-    const int c = (int)(blockIdx.x * kThreads + threadIdx.x) * V;
-    if (l > levels || c >= w) return;
-    int32_t v[kCopyRows][V];
-    bool on[kCopyRows];
-#pragma unroll
-    for (int k = 0; k < kCopyRows; k++) {
-        const int r = y * kCopyRows + k;
-        // the low quadrant belongs to the next level, unless this is the last
-        on[k] = r < h && (l == levels || r >= (h >> 1) || c >= (w >> 1));
-        if (on[k]) load_run<V>(in + (long long)r * stride + c, v[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < kCopyRows; k++)
-        if (on[k]) store_run<V>(out + (long long)(y * kCopyRows + k) * stride + c, v[k]);
-}
-
-// 16-byte accesses: both rasters 16-byte aligned, row stride and half a level's
-// width multiples of 4 ints
-bool vec4(const int *a, const int *b, int stride, int half) {
-    return ((((uintptr_t)a) | ((uintptr_t)b)) & 15) == 0 && stride % 4 == 0 && half % 4 == 0;
+    if (l > levels) return;
+    const int w = X >> (l - 1), h = Y >> (l - 1), t = (int)(blockIdx.x * kThreads + threadIdx.x);
+    if (WIDE && (!NARROW || l <= vec_level))
+        copy_rows<4>(in, out, stride, w, h, y * kCopyRows, 4 * t, l == levels);
+    else
+        copy_rows<1>(in, out, stride, w, h, y * kCopyRows, t, l == levels);
 }
 
 // Launch in stream order behind the level before it: its CTAs may become
@@ -299,7 +305,7 @@ bool valid(const int *d, const int *t, int X, int Y, int levels) {
 int level(bool fwd, bool chained, const int *in, int *out, int X, int Y, int l, cudaStream_t st) {
     const int w = X >> (l - 1), h = Y >> (l - 1);
     const unsigned gy = (unsigned)((h / 2 + kPairs - 1) / kPairs);
-    const bool vec = vec4(in, out, X, w / 2);
+    const bool vec = bpc::dwt_vec4(in, out, X, w / 2);
     const int strips = vec ? w / 8 : w / 2, per = fwd ? kThreads : 30 * (kThreads / 32);
     const dim3 g((unsigned)((strips + per - 1) / per), gy);
     return check(launch(chained, g, st, fwd ? (vec ? k_fwd<4> : k_fwd<1>) : (vec ? k_inv<4> : k_inv<1>), in, out,
@@ -309,15 +315,12 @@ int level(bool fwd, bool chained, const int *in, int *out, int X, int Y, int l, 
 
 int copy_odd(bool chained, const int *in, int *out, int X, int Y, int levels, cudaStream_t st) {
     unsigned gy = 0;
-    bool vec = true;
-    for (int l = 1; l <= levels; l += 2) {
-        gy += (unsigned)(((Y >> (l - 1)) + kCopyRows - 1) / kCopyRows);
-        vec = vec && vec4(in, out, X, (X >> (l - 1)) / 2);
-    }
-    const int per = kThreads * (vec ? 4 : 1);
+    for (int l = 1; l <= levels; l += 2) gy += (unsigned)(((Y >> (l - 1)) + kCopyRows - 1) / kCopyRows);
+    const int vec_level = bpc::dwt_copy_vec_level(in, out, X, levels), per = bpc::dwt_copy_columns(vec_level);
     const dim3 g((unsigned)((X + per - 1) / per), gy);
-    return check(launch(chained, g, st, vec ? k_copy_odd<4> : k_copy_odd<1>, in, out, (long long)X, X, Y, levels),
-                 "launch");
+    const auto kernel = vec_level == 0 ? k_copy_odd<false, true>
+                        : vec_level + 2 > levels ? k_copy_odd<true, false> : k_copy_odd<true, true>;
+    return check(launch(chained, g, st, kernel, in, out, (long long)X, X, Y, levels, vec_level), "launch");
 }
 
 }  // namespace
