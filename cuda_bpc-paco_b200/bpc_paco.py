@@ -249,6 +249,8 @@ class Batch:
         L.bpc_batch_codeblocks.restype = ctypes.c_longlong
         L.bpc_batch_words.argtypes = [vp]
         L.bpc_batch_words.restype = ctypes.c_longlong
+        L.bpc_batch_items.argtypes = [vp]
+        L.bpc_batch_items.restype = ctypes.c_longlong
         L.bpc_batch_encode.argtypes = [vp, ctypes.POINTER(vp), vp, vp, vp, vp]
         L.bpc_batch_decode.argtypes = [vp, vp, vp, ctypes.POINTER(vp), vp, vp]
         L.bpc_batch_set_schedule.argtypes = [vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int]
@@ -297,6 +299,10 @@ class Batch:
         a, b, c, d = (ctypes.c_int() for _ in range(4))
         lib().bpc_batch_get_schedule(self.h, ctypes.byref(a), ctypes.byref(b), ctypes.byref(c), ctypes.byref(d))
         return a.value, b.value, c.value, bool(d.value)
+
+    def items(self) -> int:
+        """Work items of the current schedule."""
+        return lib().bpc_batch_items(self.h)
 
     def set_tuning(self, warps_enc: int = 4, warps_dec: int = 4, cost_enc: bool = False, cost_dec: bool = False,
                    seq_enc: bool = False, seq_dec: bool = False):

@@ -257,7 +257,6 @@ namespace {
         }                                                                                 \
     } while (0)
 
-constexpr long long kItemsPerWarp = 64;  // items a warp should find before they become longer than one codeblock
 constexpr int kClasses = 4;  // (passes 2|3) x (codeblock 64|32)
 inline int class_of(int passes, int cb) { return (passes == 3 ? 2 : 0) + (cb == 32 ? 1 : 0); }
 
@@ -286,8 +285,13 @@ struct Batch {
     void *d_scan_tmp = nullptr;
     size_t scan_tmp_bytes = 0;
     int sms = 148;
-    // schedule
-    int ctas_enc = kBatchCtasEnc, ctas_dec = kBatchCtasDec, per_item = 4, use_graph = 1;
+    // schedule.  One codeblock (pair of 32x32) per item unless the caller asks
+    // for more: longer runs save queue accesses, but a warp codes a run one after
+    // the other, and the codeblocks of a coarse subband are all heavy (1 / 2 / 4
+    // / 8 per item, encode + decode: 24 mixed images, 26,655 codeblocks, 1.91 /
+    // 2.18 / 3.41 / 5.2 ms; 9 of 16384x16384, 589,824, 77.0 / 77.3 / 77.8 / 78.7;
+    // 17 of them, 1,114,112, 93.7 / 93.8 / 94.1 / 94.7).
+    int ctas_enc = kBatchCtasEnc, ctas_dec = kBatchCtasDec, per_item = 1, use_graph = 1;
     int warps_enc = kWarps, warps_dec = kWarps;  // warps per CTA: 2, 4 or 8
     int cost_enc = 0, cost_dec = 0;              // queue order: 0 coarse subbands first, 1 cost order
     int seq_enc = 0, seq_dec = 0;                // class kernels: 0 concurrent (forked streams), 1 one after another
@@ -308,17 +312,10 @@ int build_items(Batch &b) {
         int weight;
     };
     std::vector<Tmp> tmp[kClasses];
-    // A warp codes the codeblocks of an item one after the other, and those of
-    // a coarse subband are all heavy, so runs only pay (fewer queue accesses)
-    // where every warp has many items; a batch that has not gets shorter ones
-    // (24 images, 13,600 codeblocks, at most 4 / 2 / 1 per item: encode 1.35 /
-    // 1.01 / 0.96 ms, decode 2.19 / 1.19 / 0.95 ms).
-    const long long warps = (long long)b.sms * kResidentWarpsDec;
-    const int run = (int)std::max(1ll, std::min((long long)b.per_item, b.ncb / (kItemsPerWarp * warps)));
     for (int i = 0; i < b.n; i++) {
         const int cbs = b.cb[i], ncbx = b.X[i] / cbs, ncb = ncbx * (b.Y[i] / cbs);
         const int ng = cbs == 64 ? 1 : 2;
-        const int step = std::max(ng, (run + ng - 1) / ng * ng);
+        const int step = std::max(ng, (b.per_item + ng - 1) / ng * ng);
         for (int k = 0; k < ncb; k += step) {
             // coarse subbands first: level of the run's first codeblock
             const int x = (k % ncbx) * cbs, y = (k / ncbx) * cbs;
@@ -719,6 +716,13 @@ int bpc_batch_get_schedule(const void *batch, int *ctas_per_sm_enc, int *ctas_pe
     return BPC_OK;
 }
 
+long long bpc_batch_items(const void *batch) {
+    if (!batch) return BPC_ERR_ARG;
+    long long n = 0;
+    for (int c = 0; c < kClasses; c++) n += ((const Batch *)batch)->nitems[c];
+    return n;
+}
+
 int bpc_batch_encode(void *batch, const int *const *d_coeffs, int *d_compact, long long *d_offsets, int *d_status,
                      void *stream) {
     Batch *b = (Batch *)batch;
@@ -786,7 +790,11 @@ int bpc_batch_tune(void *batch, const int *const *d_coeffs, int *d_compact, long
         ms = best_run;
         return BPC_OK;
     };
+    long long last = -1;
     for (int it : items) {
+        if (const int rc = bpc_batch_set_schedule(batch, b->ctas_enc, b->ctas_dec, it, b->use_graph)) return rc;
+        if (bpc_batch_items(batch) == last) continue;  // the items of the candidate before (32x32 pairs)
+        last = bpc_batch_items(batch);
         float te_best = 1e30f, td_best = 1e30f;
         int ce = kBatchCtasEnc, cd = kBatchCtasDec;
         for (int c = 1; c <= kBatchCtasEnc; c++) {

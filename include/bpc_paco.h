@@ -168,12 +168,14 @@ int bpc_batch_encode(void *batch, const int *const *d_coeffs, int *d_compact, lo
 int bpc_batch_decode(void *batch, const int *d_compact, const long long *d_offsets, int *const *d_coeffs,
                      int *d_status, void *stream);
 /* Schedule: CTAs per SM for the encoder (1..4) and decoder (1..7), codeblocks
- * per work item (at most: a batch too small to give every warp many items uses
- * shorter ones), CUDA graph on/off.  bpc_batch_tune times the candidates on the
- * given buffers and keeps the fastest. */
+ * per work item (1..64, 1 by default; rounded up to pairs for 32x32 codeblocks),
+ * CUDA graph on/off.  bpc_batch_tune times the candidates on the
+ * given buffers and keeps the fastest.  bpc_batch_items: work items of the
+ * current schedule, all classes together. */
 int bpc_batch_set_schedule(void *batch, int ctas_per_sm_enc, int ctas_per_sm_dec, int cbs_per_item, int use_graph);
 int bpc_batch_get_schedule(const void *batch, int *ctas_per_sm_enc, int *ctas_per_sm_dec, int *cbs_per_item,
                            int *use_graph);
+long long bpc_batch_items(const void *batch);
 /* Further schedule dimensions, per direction: warps per CTA of the persistent
  * kernels (2, 4 or 8; CTAs per SM times warps per CTA may not exceed 16 for the
  * encoder and 28 for the decoder, and bpc_batch_set_tuning lowers the CTAs per
