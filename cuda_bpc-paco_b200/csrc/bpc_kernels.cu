@@ -84,8 +84,8 @@ __device__ __forceinline__ void stage_lut(const Params &p, uint8_t *tab) {
     if (bad && p.status) atomicOr(p.status, ST_LUT_RANGE);
 }
 
-// WARPS codeblock warps per CTA: kWarps, or 1 for decodes of at most one wave
-// (their heaviest codeblocks then land on different SMs, see launch_t); the
+// WARPS codeblock warps per CTA: kWarps, or 1 for small decodes (their heaviest
+// codeblocks then land on different SMs, see one_warp_pays); the
 // register budget stays that of kMinCtas x kWarps resident warps per SM
 template <int PASSES, int CBS, bool ENC, int WARPS = kWarps, int LAT = 0>
 __global__ void __launch_bounds__(WARPS * 32, (ENC ? kMinCtasEnc : kMinCtasDec) * kWarps / WARPS) k_bpc(Params p) {
@@ -276,23 +276,21 @@ static cudaError_t launch_t(const Params &p, int grid, cudaStream_t st, bool lat
     if constexpr (ENC) {
         return launch_w<PASSES, CBS, ENC, kWarps, 0>(p, grid, warps_needed, st);
     } else {
-        const long long resident = resident_warps(ENC, -1);
         // A work-ordered whole image the planner marked for isolation (p.ctr
-        // set) runs its heaviest codeblocks on SMs of their own.  Other decodes
-        // of at most one wave of resident warps run one warp per CTA, in the
-        // latency form of the step: consecutive CTAs go to different SMs, so
-        // the heaviest codeblocks (the coarse subbands, neighbours in raster
-        // order) do not share one, no SM gets a whole CTA more than another,
-        // and the warps that shared memory leaves waiting start as others end
-        // (3-pass decodes, 4-warp / one-warp CTAs: 2944x2944 0.387 / 0.318 ms,
-        // 3456x3456 0.404 / 0.334, 4096x4096 0.394 / 0.376).  Fuller ones keep
-        // 4-warp CTAs and the form with fewer instructions (5760x5760 0.550 /
-        // 0.568).
+        // set) runs its heaviest codeblocks on SMs of their own; other decodes
+        // take the one-warp form where it is the faster one.
         if constexpr (CBS == 64) {
             if (lat && grid <= 0 && p.order && p.ctr) return launch_iso<PASSES, CBS>(p, st);
         }
-        if (lat && grid <= 0 && !p.order && warps_needed <= resident)
-            return launch_w<PASSES, CBS, ENC, 1, 1>(p, grid, warps_needed, st);
+        if (lat && grid <= 0 && !p.order) {
+            int dev = 0;
+            const cudaError_t e = cudaGetDevice(&dev);
+            if (e != cudaSuccess) return e;
+            const long long r1 = one_warp_resident(sm_count(dev), shared_per_sm(dev),
+                                                   (long long)smem_bytes<PASSES, CBS, ENC, 1>(p));
+            if (one_warp_pays(PASSES, CBS, warps_needed, resident_warps(ENC, dev), r1))
+                return launch_w<PASSES, CBS, ENC, 1, 1>(p, grid, warps_needed, st);
+        }
         return launch_w<PASSES, CBS, ENC, kWarps, 0>(p, grid, warps_needed, st);
     }
 }

@@ -34,12 +34,41 @@ inline bool aligned_to(const void *p, unsigned a) { return ((uintptr_t)p & (uint
 // The longest table a mode has, 16 levels and 3 passes, is 19,845 entries.
 constexpr int kMaxLut = 230144;
 
+// Warps of one-warp decoder CTAs resident at once: each CTA keeps its own copy
+// of the table, so shared memory (smem_sm per SM, of which a CTA takes smem_cta
+// and kReservedSmem) may hold fewer of them than the registers do.
+constexpr long long kReservedSmem = 1024;
+inline long long one_warp_resident(int sms, long long smem_sm, long long smem_cta) {
+    const long long n = smem_sm / (smem_cta + kReservedSmem), regs = kMinCtasDec * kWarps;
+    return sms * (n < regs ? n : regs);
+}
+// Whether a plain decode of `warps` warps runs one-warp CTAs and the latency
+// form of the step, given the warps resident at once in 4-warp CTAs and in
+// one-warp ones.  One-warp CTAs go to different SMs one after another, so the
+// heaviest codeblocks (the coarse subbands, neighbours in raster order) do not
+// share one, and no SM gets a whole CTA more than another.  One-warp / 4-warp,
+// us:
+//   more than a wave of 4-warp CTAs: 5760x5760 568 / 550
+//   64x64, 3 passes, 5 levels: 2048x2048 296 / 369, 3456x3456 357 / 420; with
+//     deeper tables at 1.8, 2.0, 2.2 and 2.7 waves of one-warp CTAs 384 / 420,
+//     417 / 422, 423 / 419, 467 / 419 (noise amplitude 30; 60: 406 / 401, 437 /
+//     422, 447 / 410, 501 / 396): up to two waves
+//   32x32, 3 passes: 1024x1024 196 / 208, 2304x2304 (0.92 of a one-warp wave)
+//     214 / 219, 2560x2560 (1.14) 224 / 223, 2752x2752 (1.32) 240 / 227: up to one
+//   32x32, 2 passes: 1024x1024 142 / 141, 2304x2304 159 / 151, 2880x2880 180 /
+//     159: never
+inline bool one_warp_pays(int passes, int cbs, long long warps, long long resident4, long long resident1) {
+    if (warps > resident4) return false;
+    return cbs == 64 ? warps <= 2 * resident1 : passes == 3 && warps <= resident1;
+}
+
 // Launch the encoder (enc) or decoder over p.ncb codeblocks.  grid <= 0 picks
 // one CTA per kWarps codeblocks; a positive grid runs persistent CTAs that
-// walk the codeblocks grid-stride.  latency_forms lets a decode of a few waves
-// take the latency form of the step (and one-warp CTAs if it is small), which
-// finishes a launch alone on the GPU sooner but executes more instructions;
-// callers that run many launches at once pass false.
+// walk the codeblocks grid-stride.  latency_forms lets a decode take one-warp
+// CTAs and the latency form of the step (one_warp_pays; the heavy launch of an
+// isolated decode runs it too), which finish a launch alone on the GPU sooner
+// but execute more instructions; callers that run many launches at once pass
+// false.
 cudaError_t launch_code(bool enc, int passes, int cbs, const Params &p, int grid, cudaStream_t st,
                         bool latency_forms = true);
 
@@ -59,9 +88,11 @@ int code_device(bool enc, const int *in, int *out, int X, int Y, const int *d_lu
 // launch's queue counter in the scratch.  Other images keep raster order
 // (p.order and p.ctr stay null).
 long long sched_ints(int ncb, int cbs);
-// SMs of device `dev`, and its opt-in shared memory per block (cached)
+// SMs of device `dev`, its opt-in shared memory per block and its shared memory
+// per SM (cached)
 int sm_count(int dev);
 int shared_optin(int dev);
+int shared_per_sm(int dev);
 // warps of the plain coder resident at once on device `dev` (-1: current)
 int resident_warps(bool enc, int dev);
 // more than two waves on device `dev` (-1: the current device)

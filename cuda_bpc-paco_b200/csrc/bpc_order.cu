@@ -227,6 +227,11 @@ int shared_optin(int dev) {
     return cached_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin, cache, dev);
 }
 
+int shared_per_sm(int dev) {
+    static std::atomic<int> cache[64];
+    return cached_attr(cudaDevAttrMaxSharedMemoryPerMultiprocessor, cache, dev);
+}
+
 // warps resident at once on device `dev` (-1: the current device)
 int resident_warps(bool enc, int dev) {
     if (dev < 0 && cudaGetDevice(&dev) != cudaSuccess) return 1 << 30;
