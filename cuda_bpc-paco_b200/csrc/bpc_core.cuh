@@ -12,14 +12,15 @@
 //     :268-279).  That reservation order IS the bitstream.
 //
 // Representation (new): instead of one 32-bit word per coefficient with flag
-// bits (:1120), a lane keeps bit masks of its stripe and of the two neighbour
-// columns.  The encoder (bpc_enc.cuh) derives whole passes from column masks
-// bit-parallel; the decoder (bpc_dec.cuh) walks the rows with a byte of
-// neighbourhood bits per row.  Magnitudes are held as bitplanes in a per-thread
-// array built with an in-register 32x32 bit transpose; the decoder collects
-// decoded planes the same way and transposes them back at the end.  Shared
-// memory holds the LUT bytes, the sign-context table and, per warp, the
-// decoder's codeword ring and row state or the encoder's event-ranking words.
+// bits (:1120), a lane keeps bits of its stripe and of the two neighbour
+// columns.  The encoder (bpc_enc.cuh) keeps words of 16 rows in scan order, both
+// columns interleaved, and derives whole passes from them bit-parallel; the
+// decoder (bpc_dec.cuh) walks the rows with a byte of neighbourhood bits per
+// row.  Magnitudes are held as bitplanes in a per-thread array built with an
+// in-register 32x32 bit transpose; the decoder collects decoded planes the same
+// way and transposes them back at the end.  Shared memory holds the LUT bytes,
+// the sign-context table and, per warp, the decoder's codeword window and row
+// state or the encoder's event-ranking words and symbol descriptors.
 //
 // The code is written against a small warp interface W (lane id, ballot, any,
 // shuffles, syncwarp) so the same source runs as a CUDA kernel (bpc_kernels.cu)
@@ -161,7 +162,6 @@ struct Geo {
     // refinement sets, SPP-coded marks
     static constexpr int ROW_WORDS = CBS / 4 * 32, REF_WORDS = CBS / 16 * 32, VIS_WORDS = CBS / 4 * 8;
     static constexpr int RING_WORDS = RING * NG + ROW_WORDS + REF_WORDS + VIS_WORDS;  // per warp
-    static constexpr uint64_t ROWS = CBS == 64 ? ~0ull : 0xffffffffull;
 };
 
 BPC_FI int popc32(uint32_t x) {
@@ -169,13 +169,6 @@ BPC_FI int popc32(uint32_t x) {
     return __popc(x);
 #else
     return __builtin_popcount(x);
-#endif
-}
-BPC_FI int popc64(uint64_t x) {
-#if defined(__CUDA_ARCH__)
-    return __popcll(x);
-#else
-    return __builtin_popcountll(x);
 #endif
 }
 BPC_FI void add_u64(unsigned long long *p, unsigned long long v) {
@@ -224,8 +217,6 @@ BPC_FI void transpose32(uint32_t a[32]) {
     }
 }
 
-BPC_FI uint32_t bit64(uint64_t m, int i) { return (uint32_t)(m >> i) & 1u; }
-
 BPC_FI uint32_t funnel_r(uint32_t lo, uint32_t hi, int n) {
 #if defined(__CUDA_ARCH__)
     return __funnelshift_r(lo, hi, n);
@@ -248,40 +239,11 @@ BPC_FI uint32_t perm8(uint32_t v, uint32_t sel) {
 #endif
 }
 
-// Interleave the low 16 bits of a (even positions) and b (odd positions):
-// row j of the left column -> bit 2j, of the right column -> bit 2j+1, which
-// is the scan order of one lane's two columns.
-BPC_FI uint32_t spread16(uint32_t x) {
-    x &= 0xFFFFu;
-    x = (x | (x << 8)) & 0x00FF00FFu;
-    x = (x | (x << 4)) & 0x0F0F0F0Fu;
-    x = (x | (x << 2)) & 0x33333333u;
-    x = (x | (x << 1)) & 0x55555555u;
-    return x;
-}
-BPC_FI uint32_t zip16(uint64_t l, uint64_t r, int q) {
-    return spread16((uint32_t)(l >> (16 * q))) | (spread16((uint32_t)(r >> (16 * q))) << 1);
-}
-
-// Per-row count (0..8) of eight 64-bit row masks, as four bit slices
-// (carry-save adder tree; bit i of slice k = bit k of the count at row i).
-BPC_FI void count8(const uint64_t x[8], uint64_t &c0, uint64_t &c1, uint64_t &c2, uint64_t &c3) {
-    const uint64_t s1 = x[0] ^ x[1] ^ x[2], k1 = (x[0] & x[1]) | (x[2] & (x[0] ^ x[1]));
-    const uint64_t s2 = x[3] ^ x[4] ^ x[5], k2 = (x[3] & x[4]) | (x[5] & (x[3] ^ x[4]));
-    const uint64_t s3 = x[6] ^ x[7], k3 = x[6] & x[7];
-    c0 = s1 ^ s2 ^ s3;
-    const uint64_t k4 = (s1 & s2) | (s3 & (s1 ^ s2));  // weight 2
-    const uint64_t t = k1 ^ k2 ^ k3, k5 = (k1 & k2) | (k3 & (k1 ^ k2));  // weight 2 / 4
-    c1 = t ^ k4;
-    const uint64_t k6 = t & k4;  // weight 4
-    c2 = k5 ^ k6;
-    c3 = k5 & k6;
-}
-
 // Size of the encoder's per-lane event array (8-byte aligned): two words per
 // reservation of one pass.  There is at most one reservation per symbol call,
 // and a lane makes at most two calls per coefficient of its stripe (256 for
-// 64x64, 128 for 32x32).  kEvKeys: no second array is needed.
+// 64x64, 128 for 32x32).  kEvKeys: the constructor's byte array, which no coder
+// uses any more.
 constexpr int kEvKeys = 1, kEvVals = 512;
 
 // Decoder codeword window: lane gl of a codeblock's lane group fills its share
@@ -319,17 +281,6 @@ BPC_NOINLINE void ring_fill(uint32_t *ring, const int32_t *slot_in, uint32_t in_
     }
 #pragma unroll
     for (int q = 0; q < per; q++) ring[(q & ~3) * G::NL + 4 * gl + (q & 3)] = v[q];
-}
-
-template <class W>
-BPC_FI uint64_t shfl_up64(W &w, uint64_t v) {
-    uint32_t lo = w.shfl_up((uint32_t)v, 1), hi = w.shfl_up((uint32_t)(v >> 32), 1);
-    return ((uint64_t)hi << 32) | lo;
-}
-template <class W>
-BPC_FI uint64_t shfl_down64(W &w, uint64_t v) {
-    uint32_t lo = w.shfl_down((uint32_t)v, 1), hi = w.shfl_down((uint32_t)(v >> 32), 1);
-    return ((uint64_t)hi << 32) | lo;
 }
 
 // LAT > 0 selects the decoder's latency form, for launches whose time is the

@@ -33,17 +33,9 @@ struct GpuWarp {
         a = v.x;
         b = v.y;
     }
-    __device__ __forceinline__ int32_t load1(const int32_t *p) { return __ldg(p); }
     __device__ __forceinline__ void store1(int32_t *p, int32_t a) { *p = a; }
     __device__ __forceinline__ void store2(int32_t *p, int32_t a, int32_t b) {
         *reinterpret_cast<int2 *>(p) = make_int2(a, b);
-    }
-    __device__ __forceinline__ void load4(const int32_t *p, uint32_t &a, uint32_t &b, uint32_t &c, uint32_t &d) {
-        const int4 v = __ldg(reinterpret_cast<const int4 *>(p));
-        a = (uint32_t)v.x;
-        b = (uint32_t)v.y;
-        c = (uint32_t)v.z;
-        d = (uint32_t)v.w;
     }
     __device__ __forceinline__ void atomic_or(int *p, int v) { atomicOr(p, v); }
 };
