@@ -40,10 +40,11 @@ struct GpuWarp {
     __device__ __forceinline__ void atomic_or(int *p, int v) { atomicOr(p, v); }
 };
 
-// The LUT's first tab_n entries as bytes in shared memory (zeros where it is
-// shorter); entries outside 0..255, also past tab_n, are flagged and read as 0.  Four entries per load and several loads in
-// flight per thread: a CTA starts with this, and one load after another it took
-// 10-15 us of a small image's time (one-warp CTAs, 6480 entries).
+// The LUT as bytes in shared memory, zero-padded to tab_n (lut_n is at most that
+// here, see launch_code); entries outside 0..255 are flagged and read as 0.  Four
+// entries per load and several loads in flight per thread: a CTA starts with
+// this, and one load after another it took 10-15 us of a small image's time
+// (one-warp CTAs, 6480 entries).
 __device__ __forceinline__ void stage_lut(const Params &p, uint8_t *tab) {
     int bad = 0;
     const bool vec = ((uintptr_t)p.lut & 15u) == 0u;
@@ -59,19 +60,17 @@ __device__ __forceinline__ void stage_lut(const Params &p, uint8_t *tab) {
             v.z = (unsigned)v.z > 255u ? 0 : v.z;
             v.w = (unsigned)v.w > 255u ? 0 : v.w;
         }
-        if (4 * k < p.tab_n)  // tab_n is a multiple of 16
-            reinterpret_cast<uchar4 *>(tab)[k] =
-                make_uchar4((unsigned char)v.x, (unsigned char)v.y, (unsigned char)v.z, (unsigned char)v.w);
+        reinterpret_cast<uchar4 *>(tab)[k] =
+            make_uchar4((unsigned char)v.x, (unsigned char)v.y, (unsigned char)v.z, (unsigned char)v.w);
     }
-    const int end = p.lut_n > p.tab_n ? p.lut_n : p.tab_n;
 #pragma unroll 4
-    for (int k = 4 * n4 + (int)threadIdx.x; k < end; k += (int)blockDim.x) {
+    for (int k = 4 * n4 + (int)threadIdx.x; k < p.tab_n; k += (int)blockDim.x) {
         int v = k < p.lut_n ? __ldg(p.lut + k) : 0;
         if (v < 0 || v > 255) {
             bad = 1;
             v = 0;
         }
-        if (k < p.tab_n) tab[k] = (uint8_t)v;
+        tab[k] = (uint8_t)v;
     }
     if (bad && p.status) atomicOr(p.status, ST_LUT_RANGE);
 }
@@ -287,10 +286,27 @@ static cudaError_t launch_t(const Params &p, int grid, cudaStream_t st, bool lat
     }
 }
 
-cudaError_t launch_code(bool enc, int passes, int cbs, const Params &p, int grid, cudaStream_t st, bool lat) {
+// The entries of a LUT that is longer than its mode's table: range check only.
+// A kernel of its own: with the test in stage_lut the decoder's code comes out
+// differently and its chain 3-5 % longer (2048x2048, 3 passes 284 -> 297 us).
+__global__ void k_lut_rest(const int *lut, int begin, int end, int *status) {
+    const int k = begin + (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (k < end && (lut[k] < 0 || lut[k] > 255)) atomicOr(status, ST_LUT_RANGE);
+}
+
+cudaError_t launch_code(bool enc, int passes, int cbs, const Params &params, int grid, cudaStream_t st, bool lat) {
+    Params p = params;
     if (p.cb_end <= p.cb_begin) return cudaSuccess;
     if (p.lut_n > kMaxLut) return cudaErrorInvalidValue;
     if (enc) {
+    if (p.lut_n > p.tab_n) {
+        if (p.status) {
+            k_lut_rest<<<(p.lut_n - p.tab_n + 255) / 256, 256, 0, st>>>(p.lut, p.tab_n, p.lut_n, p.status);
+            const cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess) return e;
+        }
+        p.lut_n = p.tab_n;
+    }
         if (passes == 2)
             return cbs == 64 ? launch_t<2, 64, true>(p, grid, st, lat) : launch_t<2, 32, true>(p, grid, st, lat);
         return cbs == 64 ? launch_t<3, 64, true>(p, grid, st, lat) : launch_t<3, 32, true>(p, grid, st, lat);

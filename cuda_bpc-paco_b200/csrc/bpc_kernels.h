@@ -30,7 +30,7 @@ constexpr int kMinCtasEnc = ENC_MIN_CTAS;
 constexpr unsigned kEncInAlign = 8, kDecInAlign = 16;
 inline bool aligned_to(const void *p, unsigned a) { return ((uintptr_t)p & (uintptr_t)(a - 1)) == 0; }
 
-// Longest LUT a launch takes (every CTA reads all of it, for the range check).
+// Longest LUT a launch takes; entries past Params::tab_n are range-checked only.
 // The longest table a mode has, 16 levels and 3 passes, is 19,845 entries.
 constexpr int kMaxLut = 230144;
 
