@@ -47,19 +47,22 @@ inline long long one_warp_resident(int sms, long long smem_sm, long long smem_ct
 // one-warp ones.  One-warp CTAs go to different SMs one after another, so the
 // heaviest codeblocks (the coarse subbands, neighbours in raster order) do not
 // share one, and no SM gets a whole CTA more than another.  One-warp / 4-warp,
-// us:
+// us, images of noise amplitude 30 and 60:
 //   more than a wave of 4-warp CTAs: 5760x5760 568 / 550
-//   64x64, 3 passes, 5 levels: 2048x2048 296 / 369, 3456x3456 357 / 420; with
-//     deeper tables at 1.8, 2.0, 2.2 and 2.7 waves of one-warp CTAs 384 / 420,
-//     417 / 422, 423 / 419, 467 / 419 (noise amplitude 30; 60: 406 / 401, 437 /
-//     422, 447 / 410, 501 / 396): up to two waves
-//   32x32, 3 passes: 1024x1024 196 / 208, 2304x2304 (0.92 of a one-warp wave)
-//     214 / 219, 2560x2560 (1.14) 224 / 223, 2752x2752 (1.32) 240 / 227: up to one
-//   32x32, 2 passes: 1024x1024 142 / 141, 2304x2304 159 / 151, 2880x2880 180 /
-//     159: never
+//   64x64, 3 passes: 2560x2560 310 / 376 and 312 / 383, 3456x3456 342 / 414 and
+//     353 / 396; with deeper tables at 1.8 waves of one-warp CTAs 371 / 415 and
+//     394 / 395, at 2.0 403 / 418 and 416 / 418, at 2.2 408 / 413 and 432 / 405, at
+//     2.7 443 / 414 and 477 / 394: up to two waves
+//   32x32, 3 passes: 1024x1024 196 / 206 and 191 / 200, 2304x2304 (0.92 of a
+//     one-warp wave) 214 / 216 and 206 / 210, 2752x2752 (1.32) 229 / 229 and 244 /
+//     222: up to one
+//   32x32, 2 passes: 1024x1024 136 / 138 and 134 / 136, 1536x1536 (0.28 of a
+//     4-warp wave) 141 / 140 and 139 / 138, 2560x2560 153 / 150 and 163 / 157,
+//     2880x2880 179 / 157 and 186 / 171: up to a quarter of a 4-warp wave
 inline bool one_warp_pays(int passes, int cbs, long long warps, long long resident4, long long resident1) {
     if (warps > resident4) return false;
-    return cbs == 64 ? warps <= 2 * resident1 : passes == 3 && warps <= resident1;
+    if (cbs == 64) return warps <= 2 * resident1;
+    return passes == 3 ? warps <= resident1 : 4 * warps <= resident4 && warps <= resident1;
 }
 
 // Launch the encoder (enc) or decoder over p.ncb codeblocks.  grid <= 0 picks
