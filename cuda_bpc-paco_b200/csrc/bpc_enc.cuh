@@ -61,6 +61,7 @@ struct Coder<PASSES, CBS, true, W, LAT> {
     uint32_t cnt;   // codewords reserved in this codeblock (group-uniform)
     int open_slot;  // slot of the lane's last reservation (-1: none yet)
     int nev;        // events of the pass
+    bool one_group;  // LUT statistics: the lanes of each codeblock share a subband (warp-uniform)
     // stripe state: significance, signs and their outer neighbours, significant
     // at the plane's start, pending for CP, the plane's bits
     uint32_t S[NQ], N[NQ], H[NQ], HN[NQ], R[NQ], C[NQ], B[NQ];
@@ -360,18 +361,22 @@ struct Coder<PASSES, CBS, true, W, LAT> {
             P4 = (uint32_t)sp[0] | ((uint32_t)sp[1] << 8) | ((uint32_t)sp[2] << 16) | ((uint32_t)sp[3] << 24);
         }
         uint32_t above[4] = {0u, 0u, 0u, 0u}, here[2];
+        [[maybe_unused]] uint32_t c[13] = {};
         add3(S[0], inner(S[0]), H[0], here[0], here[1]);
 #pragma unroll 1
         for (int q = 0; q < NQ; q++) {
             uint32_t x[8];
             slices(q, above, here, x);
-            if (STATS)
-                stats_word(st, sig_b, sign_b, b, x);
-            else
+            if (!STATS)
                 code_word(q, x, sig_b, P4);
+            else if (b < 15)
+                stats_word(c, x);
             rotate(S), rotate(N), rotate(H), rotate(HN), rotate(NS), rotate(HNS), rotate(K);
         }
-        if (!STATS) rank_events();
+        if (!STATS)
+            rank_events();
+        else if (b < 15)
+            stats_store(st, sig_b, sign_b, c);
 #pragma unroll
         for (int q = 0; q < NQ; q++) {
             S[q] |= NS[q];
@@ -386,7 +391,14 @@ struct Coder<PASSES, CBS, true, W, LAT> {
             uint32_t n = 0, ones = 0;
 #pragma unroll
             for (int q = 0; q < NQ; q++) n += (uint32_t)popc32(R[q]), ones += (uint32_t)popc32(R[q] & B[q]);
-            if (act && b < 15) tally(st, g + b, n, ones);
+            if (b >= 15) return;
+            if (!act) n = ones = 0;
+            uint32_t v = n | (ones << 16);
+            if (one_group) {
+                v = sum_lanes(v);
+                if (gl != 0) v = 0;
+            }
+            tally(st, g + b, v & 0xFFFFu, v >> 16);
             return;
         }
         const uint32_t P = tab[g + b];
@@ -413,19 +425,43 @@ struct Coder<PASSES, CBS, true, W, LAT> {
         if (n) add_u64(st + 2 * idx, n);
         if (ones) add_u64(st + 2 * idx + 1, ones);
     }
-    BPC_FI void stats_word(unsigned long long *st, int sig_b, int sign_b, int b, const uint32_t x[8]) {
-        if (b >= 15) return;
-#pragma unroll 1
+    // A pass's counts, 9 significance contexts and 4 sign ones: symbols in the low
+    // half of a word, 1s in the high half (at most 128 a lane, 4096 a codeblock).
+    // Atomics are what bounds this kernel, so the counts are summed over the
+    // stripe's words and, where the codeblock lies in one subband, over its
+    // lanes before they go to memory (4096x4096, 2 passes, 64x64: per word and
+    // lane 1545 us, per lane 529, per codeblock 77).
+    BPC_FI void stats_word(uint32_t c[13], const uint32_t x[8]) {
+#pragma unroll
         for (int k = 0; k < 9; k++) {
             uint32_t m = K[0];
 #pragma unroll
             for (int i = 0; i < 4; i++) m &= ((k >> i) & 1) ? x[i] : ~x[i];
-            tally(st, sig_b + k, (uint32_t)popc32(m), (uint32_t)popc32(m & NS[0]));
+            c[k] += (uint32_t)popc32(m) | ((uint32_t)popc32(m & NS[0]) << 16);
         }
-#pragma unroll 1
+#pragma unroll
         for (int k = 0; k < 4; k++) {
             const uint32_t m = NS[0] & ((k & 1) ? x[5] : ~x[5]) & ((k & 2) ? x[6] : ~x[6]);
-            tally(st, sign_b + k, (uint32_t)popc32(m), (uint32_t)popc32(m & x[7]));
+            c[9 + k] += (uint32_t)popc32(m) | ((uint32_t)popc32(m & x[7]) << 16);
+        }
+    }
+    BPC_FI uint32_t sum_lanes(uint32_t v) {
+#pragma unroll
+        for (int o = G::NL / 2; o; o >>= 1) v += w.shfl_xor(v, o);
+        return v;
+    }
+    BPC_FI void stats_store(unsigned long long *st, int sig_b, int sign_b, const uint32_t c[13]) {
+        if (one_group) {
+            uint32_t own = 0;  // lane k of the codeblock adds counter k
+#pragma unroll
+            for (int k = 0; k < 13; k++) {
+                const uint32_t v = sum_lanes(c[k]);
+                own = gl == k ? v : own;
+            }
+            if (gl < 13) tally(st, gl < 9 ? sig_b + gl : sign_b + gl - 9, own & 0xFFFFu, own >> 16);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 13; k++) tally(st, k < 9 ? sig_b + k : sign_b + k - 9, c[k] & 0xFFFFu, c[k] >> 16);
         }
     }
 
@@ -540,6 +576,7 @@ struct Coder<PASSES, CBS, true, W, LAT> {
             S[q] = N[q] = H[q] = HN[q] = 0u;
             C[q] = ~0u;  // CP flag at start (:34-39, :73-78)
         }
+        if (STATS) one_group = !w.any(g != (int)w.shfl_idx((uint32_t)g, lane & ~(G::NL - 1)));
         L = E = 0u;
         cnt = 0u;
         status = 0;
