@@ -9,11 +9,13 @@ namespace bpc {
 
 constexpr int kWarps = 4;  // warps (codeblocks) per CTA
 // CTAs per SM the register budget is sized for.  Decoder: 7 x 4 warps at 72
-// registers (a 16384x16384 3-pass decode at 6 / 7 / 8 CTAs: 5.17 / 4.87 / 4.81
+// registers, of which the 4-warp forms spill 28-48 bytes and the one-warp 64x64
+// forms none (a 16384x16384 3-pass decode at 6 / 7 / 8 CTAs: 5.17 / 4.87 / 4.81
 // ms, but a 4096x4096 one, one wave, 0.384 / 0.390 / 0.404 ms).  Encoder: 5 x 4
-// warps at 102 registers (4 / 5 / 6 CTAs: 4.48 / 4.13 / 4.06 ms at 16384x16384,
-// 0.160 / 0.160 / 0.182 ms at 2048x2048, where the 6-CTA form's spills lengthen
-// the serial chain of the heaviest codeblock).
+// warps, a budget of 102 registers (64x64 takes 96, 32x32 80 and 90; no spills;
+// 4 / 5 / 6 CTAs: 4.48 / 4.13 / 4.06 ms at 16384x16384, 0.160 / 0.160 / 0.182 ms
+// at 2048x2048, where the 6-CTA form's spills lengthen the serial chain of the
+// heaviest codeblock).
 #ifndef DEC_MIN_CTAS
 #define DEC_MIN_CTAS 7
 #endif

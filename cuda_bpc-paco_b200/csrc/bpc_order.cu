@@ -39,8 +39,9 @@ constexpr int kBuckets = 1024;  // = threads of the sorting CTA
 // costs about as much as decoding 128 codewords (fit of per-codeblock decoder
 // cycles on a B200 to words + planes).  For picking the few heaviest
 // codeblocks of an isolated decode the planes weigh double: the chains that
-// end last are those of the most planes (a 4096x4096 decode with 256: 0.560
-// ms; with 128: 0.597 ms; with 64: 0.601 ms).
+// end last are those of the most planes (3-pass decodes with 64 / 128 / 256 /
+// 512: 4096x4096 386 / 372 / 361 / 362 us, a noisy 5760x5760 690 / 667 / 629 /
+// 630; 2 passes, 5120x5120 403 / 382 / 366 / 377).
 constexpr uint32_t kPlaneWords = 128, kPlaneWordsIso = 256;
 
 // Eight lanes per unit.  The first -1 is found eight probes at a time (four
@@ -120,8 +121,10 @@ __device__ __forceinline__ int cost_bin(uint32_t cost, int shift) {
 // Counting sort.  Every CTA counts the bins of all units, and apart from that
 // those of the units before its own share, and so knows where its share goes
 // without talking to the others; the loads of several rounds are in flight
-// together.  (One CTA, one load at a time: 58 us for the encoder's 65536 units,
-// 74 for the decoder's, 9 for a decoder's 4096.)
+// together.  The work grows with the square of the units, and so meets the sort
+// on one CTA only at the largest image there is (encoder / decoder, one CTA ->
+// this: 65,536 units 66 / 144 -> 38 / 17 us, 262,144 244 / 557 -> 130 / 43,
+// 1,048,576, all that 2^31 - 1 coefficients hold, 953 / 2206 -> 964 / 266).
 //
 // COARSE (encoder, a few dozen different costs): a warp's units of equal cost
 // claim their places together and stay in raster order.  Scattered one by one
