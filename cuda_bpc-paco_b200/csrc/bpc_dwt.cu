@@ -228,22 +228,33 @@ __global__ void __launch_bounds__(kThreads) k_inv(const int32_t *in, int32_t *ou
 // accesses (dwt_copy_vec_level); WIDE / NARROW: some levels do / do not (both
 // ways in every launch cost 3072x2048 1 us of 43).
 constexpr int kCopyRows = 4;
-template <int V>
-__device__ __forceinline__ void copy_rows(const int32_t *in, int32_t *out, long long stride, int w, int h, int r0, int c,
+template <bool WIDE>
+__device__ __forceinline__ void copy_rows(const int32_t *in, int32_t *out, long long stride, int w, int h, int r0, int t,
                                           bool whole) {
-    if (c >= w) return;
-    int32_t v[kCopyRows][V];
-    bool on[kCopyRows];
+    const int c0 = bpc::dwt_copy_column(WIDE, t, 0);
+    int32_t v[kCopyRows][4];
+    bool on[kCopyRows][4];
 #pragma unroll
     for (int k = 0; k < kCopyRows; k++) {
         const int r = r0 + k;
-        // the low quadrant belongs to the next level, unless this is the last
-        on[k] = r < h && (whole || r >= (h >> 1) || c >= (w >> 1));
-        if (on[k]) load_run<V>(in + (long long)r * stride + c, v[k]);
+        const int32_t *p = in + (long long)r * stride + c0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int c = bpc::dwt_copy_column(WIDE, t, j);
+            // the low quadrant belongs to the next level, unless this is the last
+            on[k][j] = r < h && c < w && (whole || r >= (h >> 1) || c >= (w >> 1));
+            if (!WIDE && on[k][j]) v[k][j] = p[j * kThreads];
+        }
+        if (WIDE && on[k][0]) load_run<4>(p, v[k]);
     }
 #pragma unroll
-    for (int k = 0; k < kCopyRows; k++)
-        if (on[k]) store_run<V>(out + (long long)(r0 + k) * stride + c, v[k]);
+    for (int k = 0; k < kCopyRows; k++) {
+        int32_t *p = out + (long long)(r0 + k) * stride + c0;
+        if (WIDE && on[k][0]) store_run<4>(p, v[k]);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (!WIDE && on[k][j]) p[j * kThreads] = v[k][j];
+    }
 }
 template <bool WIDE, bool NARROW>
 __global__ void __launch_bounds__(kThreads) k_copy_odd(const int32_t *in, int32_t *out, long long stride, int X, int Y,
@@ -258,9 +269,9 @@ __global__ void __launch_bounds__(kThreads) k_copy_odd(const int32_t *in, int32_
     if (l > levels) return;
     const int w = X >> (l - 1), h = Y >> (l - 1), t = (int)(blockIdx.x * kThreads + threadIdx.x);
     if (WIDE && (!NARROW || l <= vec_level))
-        copy_rows<4>(in, out, stride, w, h, y * kCopyRows, 4 * t, l == levels);
+        copy_rows<true>(in, out, stride, w, h, y * kCopyRows, t, l == levels);
     else
-        copy_rows<1>(in, out, stride, w, h, y * kCopyRows, t, l == levels);
+        copy_rows<false>(in, out, stride, w, h, y * kCopyRows, t, l == levels);
 }
 
 // Launch in stream order behind the level before it: its CTAs may become
@@ -316,7 +327,7 @@ int level(bool fwd, bool chained, const int *in, int *out, int X, int Y, int l, 
 int copy_odd(bool chained, const int *in, int *out, int X, int Y, int levels, cudaStream_t st) {
     unsigned gy = 0;
     for (int l = 1; l <= levels; l += 2) gy += (unsigned)(((Y >> (l - 1)) + kCopyRows - 1) / kCopyRows);
-    const int vec_level = bpc::dwt_copy_vec_level(in, out, X, levels), per = bpc::dwt_copy_columns(vec_level);
+    const int vec_level = bpc::dwt_copy_vec_level(in, out, X, levels), per = bpc::kDwtCopyColumns;
     const dim3 g((unsigned)((X + per - 1) / per), gy);
     const auto kernel = vec_level == 0 ? k_copy_odd<false, true>
                         : vec_level + 2 > levels ? k_copy_odd<true, false> : k_copy_odd<true, true>;

@@ -19,7 +19,8 @@ def plan(tmp_path_factory):
         f.write('#include "bpc_dwt_plan.h"\n'
                 'extern "C" int vec_level(long a, long b, int X, int levels) '
                 '{ return bpc::dwt_copy_vec_level((void *)a, (void *)b, X, levels); }\n'
-                'extern "C" int columns(int v) { return bpc::dwt_copy_columns(v); }\n')
+                'extern "C" int columns() { return bpc::kDwtCopyColumns; }\n'
+                'extern "C" int column(int wide, int t, int j) { return bpc::dwt_copy_column(wide, t, j); }\n')
     subprocess.check_call(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I",
                            os.path.join(ROOT, "cuda_bpc-paco_b200", "csrc"), src, "-o", out])
     L = ctypes.CDLL(out)
@@ -36,20 +37,17 @@ def test_each_level_has_its_own_accesses(plan, X, levels, want):
         assert plan.vec_level((1 << 20) + a, (3 << 20) + b, X, levels) == 0
 
 
-def test_copy_covers_every_level(plan):
-    for X in list(range(2, 1500, 2)) + list(range(8000, 8700, 2)) + [32768]:
-        for levels in range(1, 15):
-            if X % (1 << levels):
-                break
-            v = plan.vec_level(0, 0, X, levels)
-            ctas = -(-X // plan.columns(v))
-            for l in range(1, levels + 1, 2):
-                assert ctas * 128 * (4 if l <= v else 1) >= X >> (l - 1), (X, levels, l)
+@pytest.mark.parametrize("wide", [0, 1])
+def test_copy_covers_each_column_once(plan, wide):
+    for w in (2, 8, 128, 510, 512, 520, 1544, 5998):
+        threads = -(-w // plan.columns()) * 128
+        cols = sorted(plan.column(wide, t, j) for t in range(threads) for j in range(4))
+        assert cols == list(range(threads * 4)) and threads * 4 >= w
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("H,W,levels", [(96, 320, 5), (64, 1984, 5), (128, 8256, 5), (40, 264, 3), (32, 4112, 4),
-                                        (64, 96, 5)])
+                                        (64, 96, 5), (34, 1030, 1), (36, 1500, 2), (30, 514, 1)])
 def test_mixed_accesses(bpc, H, W, levels):
     import torch
     rng = np.random.default_rng(W + levels)
