@@ -9,7 +9,7 @@ namespace bpc {
 
 constexpr int kWarps = 4;  // warps (codeblocks) per CTA
 // CTAs per SM the register budget is sized for.  Decoder: 7 x 4 warps at 72
-// registers, of which the 4-warp forms spill 28-48 bytes and the one-warp 64x64
+// registers, of which the 4-warp forms spill 16-40 bytes and the one-warp 64x64
 // forms none (a 16384x16384 3-pass decode at 6 / 7 / 8 CTAs: 5.17 / 4.87 / 4.81
 // ms, but a 4096x4096 one, one wave, 0.384 / 0.390 / 0.404 ms).  Encoder: 5 x 4
 // warps, a budget of 102 registers (64x64 takes 96, 32x32 80 and 90; no spills;
